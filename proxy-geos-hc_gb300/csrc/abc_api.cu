@@ -189,9 +189,9 @@ int sem_mlp_set_params(sem_mlp *m, const float *params)
     if (!m || !params) return sem_fail(SEM_ERR_ARG, "NULL argument");
     for (int i = 0; i < kMlpParams; i++)
         if (!std::isfinite(params[i])) return sem_fail(SEM_ERR_ARG, "non-finite parameter");
-    CUDA_TRY(cudaMemcpy(m->d_master, params, kMlpParams * 4, cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemset(m->d_m, 0, kMlpParams * 4));
-    CUDA_TRY(cudaMemset(m->d_v, 0, kMlpParams * 4));
+    CUDA_TRY(cudaMemcpyAsync(m->d_master, params, kMlpParams * 4, cudaMemcpyHostToDevice, m->stream));
+    CUDA_TRY(cudaMemsetAsync(m->d_m, 0, kMlpParams * 4, m->stream));
+    CUDA_TRY(cudaMemsetAsync(m->d_v, 0, kMlpParams * 4, m->stream));
     m->adam_t = 0;
     return net_upload(m);
     GUARD_END
@@ -421,9 +421,10 @@ int sem_abc_reset(sem_abc *a)
 {
     GUARD_BEGIN
     if (!a) return sem_fail(SEM_ERR_ARG, "NULL boundary");
-    CUDA_TRY(cudaStreamSynchronize(a->s->stream));
-    CUDA_TRY(cudaMemset(a->d_hist, 0, (size_t)a->s->mesh->box.n_int * 4));
-    if (a->d_hist_alt) CUDA_TRY(cudaMemset(a->d_hist_alt, 0, (size_t)a->s->mesh->box.n_int * 4));
+    // on the solver's stream, ordered with the steps (see sem_solver_reset)
+    cudaStream_t st = a->s->stream;
+    CUDA_TRY(cudaMemsetAsync(a->d_hist, 0, (size_t)a->s->mesh->box.n_int * 4, st));
+    if (a->d_hist_alt) CUDA_TRY(cudaMemsetAsync(a->d_hist_alt, 0, (size_t)a->s->mesh->box.n_int * 4, st));
     a->hcur = 0;
     return SEM_OK;
     GUARD_END

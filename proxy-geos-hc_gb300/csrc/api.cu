@@ -1094,12 +1094,13 @@ int sem_solver_reset(sem_solver *s)
 {
     GUARD_BEGIN
     if (!s) return fail(SEM_ERR_ARG, "NULL solver");
-    CUDA_TRY(cudaStreamSynchronize(s->stream));
-    for (auto p : s->d_p) CUDA_TRY(cudaMemset(p, 0, s->n_int * 4));
-    if (s->d_y) CUDA_TRY(cudaMemset(s->d_y, 0, s->n_int * 4));
-    CUDA_TRY(cudaMemset(s->d_ctr, 0, 8));
-    CUDA_TRY(cudaMemset(s->d_status, 0, 4));
-    if (s->d_traces) CUDA_TRY(cudaMemset(s->d_traces, 0, (size_t)s->trace_cap * s->nrec * 4));
+    // on the solver's own stream, which does not wait for the default stream: a step enqueued
+    // after this call starts from the zeroed levels and step counter
+    for (auto p : s->d_p) CUDA_TRY(cudaMemsetAsync(p, 0, s->n_int * 4, s->stream));
+    if (s->d_y) CUDA_TRY(cudaMemsetAsync(s->d_y, 0, s->n_int * 4, s->stream));
+    CUDA_TRY(cudaMemsetAsync(s->d_ctr, 0, 8, s->stream));
+    CUDA_TRY(cudaMemsetAsync(s->d_status, 0, 4, s->stream));
+    if (s->d_traces) CUDA_TRY(cudaMemsetAsync(s->d_traces, 0, (size_t)s->trace_cap * s->nrec * 4, s->stream));
     s->steps_done = 0;
     s->traces_checked = 0;
     s->cur = 0;

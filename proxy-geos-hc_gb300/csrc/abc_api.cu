@@ -25,14 +25,15 @@ using namespace semgb;
 struct sem_mlp {
     float *d_master = nullptr;  // FP32 parameters (mlp.h layout)
     float *d_m = nullptr, *d_v = nullptr, *d_grad = nullptr;
-    float *d_part = nullptr;       // per-CTA partial gradients [kMlpMaxCTAs][kMlpParams]
-    double *d_part_loss = nullptr;  // per-CTA partial losses [kMlpMaxCTAs]
+    MlpWork work;               // training work arrays for up to work_rows rows
+    int64_t work_rows = 0;
     uint16_t *d_w1 = nullptr, *d_w2 = nullptr;
     float *d_b1 = nullptr, *d_b2 = nullptr, *d_w3 = nullptr, *d_b3 = nullptr;
     double *d_loss = nullptr;
     int adam_t = 0;
     cudaStream_t stream = nullptr;
     MlpDev dev() const { return MlpDev{d_w1, d_w2, d_b1, d_b2, d_w3, d_b3}; }
+    MlpAdam adam(float lr) { return MlpAdam{d_master, d_m, d_v, ++adam_t, lr, d_w1, d_w2, d_b1, d_b2, d_w3, d_b3}; }
 };
 
 struct sem_abc {
@@ -62,6 +63,39 @@ struct sem_abc {
 };
 
 namespace {
+
+void free_work(sem_mlp *m)
+{
+    MlpWork &w = m->work;
+    dfree(w.xb); dfree(w.h1); dfree(w.dz1); dfree(w.dz2); dfree(w.g2); dfree(w.err); dfree(w.dy); dfree(w.part);
+    dfree(w.lsum);
+    m->work_rows = 0;
+}
+
+// Training work arrays for a pass over n rows (kept with the network: at most 86 MB; passes over
+// more rows run in rounds).  The caller's stream is idle or about to use them.
+cudaError_t ensure_work(sem_mlp *m, int64_t n)
+{
+    const int64_t rows = mlp_work_rows(n);
+    if (rows <= m->work_rows) return cudaSuccess;
+    free_work(m);
+    MlpWork &w = m->work;
+    const size_t r = (size_t)rows, slots = r / kMlpTile;
+    cudaError_t e = dalloc(&w.xb, r * kMlpXbStride);
+    if (e == cudaSuccess) e = dalloc(&w.h1, r * kMlpHidden);
+    for (float **p : {&w.dz1, &w.dz2, &w.g2})
+        if (e == cudaSuccess) e = dalloc(p, r * kMlpHidden);
+    if (e == cudaSuccess) e = dalloc(&w.err, r);
+    if (e == cudaSuccess) e = dalloc(&w.dy, r);
+    if (e == cudaSuccess) e = dalloc(&w.part, slots * kMlpParams);
+    if (e == cudaSuccess) e = dalloc(&w.lsum, slots * 32);
+    if (e != cudaSuccess) {
+        free_work(m);
+        return e;
+    }
+    m->work_rows = rows;
+    return cudaSuccess;
+}
 
 int net_upload(sem_mlp *m)
 {
@@ -132,7 +166,7 @@ int sem_mlp_destroy(sem_mlp *m)
     if (!m) return SEM_OK;
     if (m->stream) cudaStreamSynchronize(m->stream);
     dfree(m->d_master); dfree(m->d_m); dfree(m->d_v); dfree(m->d_grad);
-    dfree(m->d_part); dfree(m->d_part_loss);
+    free_work(m);
     dfree(m->d_w1); dfree(m->d_w2); dfree(m->d_b1); dfree(m->d_b2); dfree(m->d_w3); dfree(m->d_b3);
     dfree(m->d_loss);
     if (m->stream) cudaStreamDestroy(m->stream);
@@ -151,8 +185,7 @@ int sem_mlp_create(uint64_t seed, sem_mlp **out)
     if (e == cudaSuccess) e = dalloc(&m->d_m, kMlpParams);
     if (e == cudaSuccess) e = dalloc(&m->d_v, kMlpParams);
     if (e == cudaSuccess) e = dalloc(&m->d_grad, kMlpParams);
-    if (e == cudaSuccess) e = dalloc(&m->d_part, (size_t)kMlpMaxCTAs * kMlpParams);
-    if (e == cudaSuccess) e = dalloc(&m->d_part_loss, (size_t)kMlpMaxCTAs);
+    if (e == cudaSuccess) e = mlp_train_setup();
     if (e == cudaSuccess) e = dalloc(&m->d_w1, kMlpHidden * kMlpInPad);
     if (e == cudaSuccess) e = dalloc(&m->d_w2, kMlpHidden * kMlpHidden);
     if (e == cudaSuccess) e = dalloc(&m->d_b1, kMlpHidden);
@@ -237,7 +270,8 @@ int sem_mlp_loss_grad(sem_mlp *m, int64_t n, const float *x, const float *t, dou
     if (e == cudaSuccess) e = cudaMemcpy(dt, t, (size_t)n * 4, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemsetAsync(m->d_grad, 0, kMlpParams * 4, m->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(m->d_loss, 0, 8, m->stream);
-    if (e == cudaSuccess) e = mlp_loss_grad(m->dev(), dx, dt, n, m->d_loss, m->d_grad, m->d_part, m->d_part_loss, m->stream);
+    if (e == cudaSuccess) e = ensure_work(m, n);
+    if (e == cudaSuccess) e = mlp_loss_grad(m->dev(), dx, dt, n, m->d_loss, m->d_grad, m->work, m->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
     if (e == cudaSuccess && loss) e = cudaMemcpy(loss, m->d_loss, 8, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess && grad) e = cudaMemcpy(grad, m->d_grad, kMlpParams * 4, cudaMemcpyDeviceToHost);
@@ -254,43 +288,54 @@ int sem_mlp_train(sem_mlp *m, int64_t n, const float *x, const float *t, int epo
     GUARD_BEGIN
     if (!m || n < 1 || !x || !t || epochs < 0 || batch < 1 || !(lr > 0))
         return sem_fail(SEM_ERR_ARG, "bad arguments");
-    // samples resident on the device, shuffled once per epoch on the host (index order)
-    float *dx = nullptr, *dt = nullptr, *bx = nullptr, *bt = nullptr;
-    const int64_t nb = std::min<int64_t>(batch, n);
-    CUDA_TRY(dalloc(&dx, (size_t)n * kMlpIn));
-    cudaError_t e = dalloc(&dt, (size_t)n);
-    if (e == cudaSuccess) e = dalloc(&bx, (size_t)nb * kMlpIn);
-    if (e == cudaSuccess) e = dalloc(&bt, (size_t)nb);
-    if (e == cudaSuccess) e = cudaMemcpy(dx, x, (size_t)n * kMlpIn * 4, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(dt, t, (size_t)n * 4, cudaMemcpyHostToDevice);
+    // samples resident on the device; their order is shuffled once per epoch on the host, while the
+    // device still runs the epoch before: two index arrays in turn, each copied on its own stream
+    const int64_t nb = std::min<int64_t>(batch, n), nbatch = n / nb;
+    float *dx = nullptr, *dt = nullptr;
+    int64_t *dperm[2] = {nullptr, nullptr};
+    double *dl = nullptr;
+    cudaStream_t copy = nullptr;
+    cudaEvent_t done[2] = {nullptr, nullptr};
+    cudaError_t e = dalloc(&dx, (size_t)n * kMlpIn);
+    if (e == cudaSuccess) e = dalloc(&dt, (size_t)n);
+    for (auto &p : dperm)
+        if (e == cudaSuccess) e = dalloc(&p, (size_t)n);
+    if (e == cudaSuccess) e = dalloc(&dl, (size_t)std::max(epochs, 1) * nbatch);
+    if (e == cudaSuccess) e = ensure_work(m, nb);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&copy, cudaStreamNonBlocking);
+    for (auto &v : done)
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&v, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(dx, x, (size_t)n * kMlpIn * 4, cudaMemcpyHostToDevice, m->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(dt, t, (size_t)n * 4, cudaMemcpyHostToDevice, m->stream);
     std::vector<int64_t> perm(n);
     for (int64_t i = 0; i < n; i++) perm[i] = i;
-    int64_t *dperm = nullptr;
-    if (e == cudaSuccess) e = dalloc(&dperm, (size_t)n);
     std::mt19937_64 rng(seed);
     for (int ep = 0; ep < epochs && e == cudaSuccess; ep++) {
         std::shuffle(perm.begin(), perm.end(), rng);
-        e = cudaMemcpyAsync(dperm, perm.data(), (size_t)n * 8, cudaMemcpyHostToDevice, m->stream);
-        double lsum = 0.0;
-        int64_t seen = 0;
-        for (int64_t b0 = 0; b0 + nb <= n && e == cudaSuccess; b0 += nb) {
-            e = mlp_gather_rows(dx, dt, dperm + b0, nb, bx, bt, m->stream);
-            if (e == cudaSuccess) e = cudaMemsetAsync(m->d_grad, 0, kMlpParams * 4, m->stream);
-            if (e == cudaSuccess) e = cudaMemsetAsync(m->d_loss, 0, 8, m->stream);
-            if (e == cudaSuccess) e = mlp_loss_grad(m->dev(), bx, bt, nb, m->d_loss, m->d_grad, m->d_part, m->d_part_loss, m->stream);
-            if (e == cudaSuccess) e = mlp_adam(m->d_master, m->d_grad, m->d_m, m->d_v, ++m->adam_t, lr, m->stream);
-            if (e == cudaSuccess)
-                e = mlp_pack(m->d_master, m->d_w1, m->d_w2, m->d_b1, m->d_b2, m->d_w3, m->d_b3, m->stream);
-            double l = 0;
-            if (e == cudaSuccess) e = cudaMemcpyAsync(&l, m->d_loss, 8, cudaMemcpyDeviceToHost, m->stream);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
-            lsum += l * nb;
-            seen += nb;
-        }
-        if (losses) losses[ep] = seen ? lsum / seen : 0.0;
+        const int k = ep & 1;
+        if (ep >= 2) e = cudaEventSynchronize(done[k]);  // the epoch that last read this index array
+        if (e == cudaSuccess) e = cudaMemcpyAsync(dperm[k], perm.data(), (size_t)n * 8, cudaMemcpyHostToDevice, copy);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(copy);
+        for (int64_t j = 0; j < nbatch && e == cudaSuccess; j++)
+            e = mlp_train_step(m->dev(), dx, dt, dperm[k] + j * nb, nb, dl + ep * nbatch + j, m->adam(lr), m->work,
+                               m->stream, j > 0);
+        if (e == cudaSuccess) e = cudaEventRecord(done[k], m->stream);
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
-    dfree(dx); dfree(dt); dfree(bx); dfree(bt); dfree(dperm);
+    const cudaError_t es = cudaStreamSynchronize(m->stream);
+    if (e == cudaSuccess) e = es;
+    if (e == cudaSuccess && losses && epochs > 0) {
+        std::vector<double> l((size_t)epochs * nbatch);
+        e = cudaMemcpy(l.data(), dl, l.size() * 8, cudaMemcpyDeviceToHost);
+        for (int ep = 0; ep < epochs; ep++) {
+            double lsum = 0.0;
+            for (int64_t j = 0; j < nbatch; j++) lsum += l[ep * nbatch + j] * nb;
+            losses[ep] = lsum / (nbatch * nb);
+        }
+    }
+    dfree(dx); dfree(dt); dfree(dperm[0]); dfree(dperm[1]); dfree(dl);
+    for (auto v : done)
+        if (v) cudaEventDestroy(v);
+    if (copy) cudaStreamDestroy(copy);
     CUDA_TRY(e);
     return SEM_OK;
     GUARD_END
@@ -301,8 +346,7 @@ int sem_mlp_adam_step(sem_mlp *m, const float *grad, float lr)
     GUARD_BEGIN
     if (!m || !grad || !(lr > 0)) return sem_fail(SEM_ERR_ARG, "bad arguments");
     CUDA_TRY(cudaMemcpyAsync(m->d_grad, grad, kMlpParams * 4, cudaMemcpyHostToDevice, m->stream));
-    CUDA_TRY(mlp_adam(m->d_master, m->d_grad, m->d_m, m->d_v, ++m->adam_t, lr, m->stream));
-    CUDA_TRY(mlp_pack(m->d_master, m->d_w1, m->d_w2, m->d_b1, m->d_b2, m->d_w3, m->d_b3, m->stream));
+    CUDA_TRY(mlp_adam(m->adam(lr), m->d_grad, m->stream));
     CUDA_TRY(cudaStreamSynchronize(m->stream));
     return SEM_OK;
     GUARD_END
@@ -521,33 +565,27 @@ int sem_abc_bptt(sem_abc *a, int n_steps, int n_roi, const int64_t *roi_nodes, c
     cudaStream_t st = s->stream;
 
     // work arrays (freed on every exit path)
-    float *rec = nullptr, *x = nullptr, *dx = nullptr, *scale = nullptr, *y = nullptr, *g = nullptr, *dy = nullptr;
+    float *rec = nullptr, *dx = nullptr;
     float *A[3] = {nullptr, nullptr, nullptr}, *v = nullptr, *dref = nullptr;
-    int *kstar = nullptr, *sidx = nullptr;
+    int *sidx = nullptr;
     int64_t *droi = nullptr;
-    double *dloss = nullptr, *dnull = nullptr;
+    double *dloss = nullptr;
     auto release = [&]() {
         cudaStreamSynchronize(st);
-        dfree(rec); dfree(x); dfree(dx); dfree(scale); dfree(y); dfree(g); dfree(dy);
+        dfree(rec); dfree(dx);
         for (auto &p : A) dfree(p);
-        dfree(v); dfree(dref); dfree(kstar); dfree(sidx); dfree(droi); dfree(dloss); dfree(dnull);
+        dfree(v); dfree(dref); dfree(sidx); dfree(droi); dfree(dloss);
     };
     cudaError_t e = dalloc(&rec, (size_t)(n_steps + 2) * n_int);
-    if (e == cudaSuccess) e = dalloc(&x, (size_t)nb * kMlpIn);
     if (e == cudaSuccess) e = dalloc(&dx, (size_t)nb * kMlpIn);
-    if (e == cudaSuccess) e = dalloc(&scale, (size_t)nb);
-    if (e == cudaSuccess) e = dalloc(&y, (size_t)nb);
-    if (e == cudaSuccess) e = dalloc(&g, (size_t)nb);
-    if (e == cudaSuccess) e = dalloc(&dy, (size_t)nb);
+    if (e == cudaSuccess && grad) e = ensure_work(a->net, nb);
     for (auto &p : A)
         if (e == cudaSuccess) e = dalloc(&p, (size_t)n_int);
     if (e == cudaSuccess) e = dalloc(&v, (size_t)n_int);
     if (e == cudaSuccess && n_roi > 0) e = dalloc(&dref, (size_t)n_steps * n_roi);
-    if (e == cudaSuccess) e = dalloc(&kstar, (size_t)nb);
     if (e == cudaSuccess) e = dalloc(&sidx, (size_t)n_int);
     if (e == cudaSuccess && n_roi > 0) e = dalloc(&droi, (size_t)n_roi);
     if (e == cudaSuccess) e = dalloc(&dloss, 1);
-    if (e == cudaSuccess) e = dalloc(&dnull, 1);
     if (e == cudaSuccess) {
         std::vector<int64_t> nodes(nb);
         e = cudaMemcpy(nodes.data(), a->d_nodes, nb * 8, cudaMemcpyDeviceToHost);
@@ -576,7 +614,7 @@ int sem_abc_bptt(sem_abc *a, int n_steps, int n_roi, const int64_t *roi_nodes, c
     f.sy = s->sponge ? s->d_sy : nullptr;
     f.sz = s->sponge ? s->d_sz : nullptr;
     f.nodes = a->d_nodes; f.nb = nb; f.sidx = sidx;
-    f.x = x; f.scale = scale; f.kstar = kstar; f.y = y; f.g = g; f.dy = dy; f.dx = dx;
+    f.dx = dx;
     for (int k = 0; k < 3; k++) f.a[k] = A[k];
     f.v = v; f.roi = droi; f.n_roi = n_roi;
     for (auto p : A)
@@ -607,12 +645,7 @@ int sem_abc_bptt(sem_abc *a, int n_steps, int n_roi, const int64_t *roi_nodes, c
             const float *lm = rec + (size_t)(m + 1) * n_int, *lm1 = rec + (size_t)m * n_int,
                         *lm2 = rec + (size_t)(m - 1) * n_int;
             e = bptt_loss(f, lm, dref + (size_t)(m - 1) * n_roi, dloss, st);
-            if (e == cudaSuccess) e = bptt_features(f, lm, lm1, lm2, st);
-            if (e == cudaSuccess) e = mlp_forward(net->dev(), x, y, nb, st);
-            if (e == cudaSuccess) e = bptt_dy(f, st);
-            if (e == cudaSuccess)
-                e = mlp_loss_grad(net->dev(), x, nullptr, nb, dnull, net->d_grad, net->d_part, net->d_part_loss, st,
-                                  dy, dx);
+            if (e == cudaSuccess) e = mlp_boundary_grad(net->dev(), f, lm, lm1, lm2, net->d_grad, net->work, st);
             if (e == cudaSuccess) e = bptt_scatter(f, st);
             if (e == cudaSuccess) e = bptt_interior(f, op, s->d_a, st);
             // the adjoints move one level back: out^{m-1} becomes the newest

@@ -8,7 +8,8 @@
 //     level 0: out_j (j not on the boundary) or s_j (s_j q_j) (j on the boundary: what the step
 //              leaves there before the network), level 1: s_j c_j, level 2: s_j q_j.
 // Backward, with A0, A1, A2 the adjoints of out^m, out^{m-1}, out^{m-2} (complete for out^m):
-//   1. g_b = A0_b; dy_b = g_b scale_b [|y_b| < 1] (N = scale h); the network's backward gives
+//   1. (mlp_boundary_grad, k_mlp_train.cu) g_b = A0_b; dy_b = g_b scale_b [|y_b| < 1] (N = scale h);
+//      the network's backward gives
 //      the parameter gradient and dx = dy dy/dx; with d = dx / scale = g dh/dx
 //      (h = clip(MLP(x)), x = f / scale) the feature gradient is
 //      G_k = d_k + [k = k*] sgn(f_k*) (g h - sum_m x_m d_m)   (scale = |f_k*|);
@@ -62,80 +63,6 @@ __device__ __forceinline__ bool inside(const Geo &g, int ix, int iy, int iz)
 __device__ __forceinline__ bool on_boundary(const Geo &g, int ix, int iy, int iz)
 {
     return ix == 0 || ix == g.nx - 1 || iy == 0 || iy == g.ny - 1 || iz == 0 || iz == g.nz - 1;
-}
-
-__global__ void k_bptt_features(const Geo g, const int64_t *nodes, int64_t nb, const float *lm, const float *lm1,
-                                const float *lm2, float *x, float *scale, int *kstar)
-{
-    for (int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += (int64_t)gridDim.x * blockDim.x) {
-        int ix, iy, iz;
-        coords_of(g, nodes[b], ix, iy, iz);
-        float f[kMlpIn];
-#pragma unroll
-        for (int nbh = 0; nbh < 27; nbh++) {
-            const int jx = ix + nbh % 3 - 1, jy = iy + (nbh / 3) % 3 - 1, jz = iz + nbh / 9 - 1;
-            float f0 = 0.f, f1 = 0.f, f2 = 0.f;
-            if (inside(g, jx, jy, jz)) {
-                const int64_t qn = index_of(g, jx, jy, jz);
-                const float sj = sponge_of(g, jx, jy, jz);
-                const float hq = lm2[qn] * sj;  // s q: the history the step keeps
-                f0 = on_boundary(g, jx, jy, jz) ? hq * sj : lm[qn];
-                f1 = lm1[qn] * sj;
-                f2 = hq;
-            }
-            f[nbh] = f0;
-            f[27 + nbh] = f1;
-            f[54 + nbh] = f2;
-        }
-        float m = 0.f;
-        int km = 0;
-        for (int k = 0; k < kMlpIn; k++)
-            if (fabsf(f[k]) > m) { m = fabsf(f[k]); km = k; }
-        const float sc = m + 1e-30f, inv = 1.f / sc;
-        float *xr = x + b * kMlpIn;
-        for (int k = 0; k < kMlpIn; k++) xr[k] = f[k] * inv;
-        scale[b] = sc;
-        // arg-max feature and its sign; -1 for an all-zero neighbourhood (N is 0 there and has
-        // no derivative: its gradient is taken as 0)
-        kstar[b] = m > 0.f ? (km | (f[km] < 0.f ? 0x100 : 0)) : -1;
-    }
-}
-
-// g_b = A0 at the boundary node; the network output's gradient dy_b = g_b scale_b where the
-// output is not clipped (the node's value is scale clip(y))
-__global__ void k_bptt_dy(const int64_t *nodes, int64_t nb, const float *a0, const float *y, const float *scale,
-                          float *g, float *dy)
-{
-    for (int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += (int64_t)gridDim.x * blockDim.x) {
-        const float gb = a0[nodes[b]];
-        g[b] = gb;
-        dy[b] = (y[b] > -1.f && y[b] < 1.f) ? gb * scale[b] : 0.f;
-    }
-}
-
-// dx (= dy dy/dx) -> feature gradient G, in place: d = dx / scale, plus the scale's share on its
-// arg-max feature
-__global__ void k_bptt_feature_grad(int64_t nb, const float *x, const float *scale, const int *kstar, const float *g,
-                                    const float *y, float *dx)
-{
-    for (int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += (int64_t)gridDim.x * blockDim.x) {
-        const float *xr = x + b * kMlpIn;
-        float *d = dx + b * kMlpIn;
-        if (kstar[b] < 0) {
-            for (int k = 0; k < kMlpIn; k++) d[k] = 0.f;
-            continue;
-        }
-        const float inv = 1.f / scale[b];
-        float xd = 0.f;
-        for (int k = 0; k < kMlpIn; k++) {
-            d[k] *= inv;
-            xd = fmaf(xr[k], d[k], xd);
-        }
-        const float h = fminf(fmaxf(y[b], -1.f), 1.f);
-        const int ks = kstar[b];
-        const float sg = (ks & 0x100) ? -1.f : 1.f;
-        d[ks & 0xff] += sg * (g[b] * h - xd);
-    }
 }
 
 // every node collects the feature gradients of the boundary nodes whose neighbourhood holds it
@@ -244,25 +171,9 @@ int blocks_for(int64_t n) { return (int)std::min<int64_t>((n + kThreads - 1) / k
 
 }  // namespace
 
-cudaError_t bptt_features(const BpttFields &f, const float *lm, const float *lm1, const float *lm2, cudaStream_t s)
-{
-    const Geo g{f.nx, f.ny, f.nz, f.nxp, f.sx, f.sy, f.sz};
-    k_bptt_features<<<blocks_for(f.nb), kThreads, 0, s>>>(g, f.nodes, f.nb, lm, lm1, lm2, f.x, f.scale, f.kstar);
-    return cudaGetLastError();
-}
-
-cudaError_t bptt_dy(const BpttFields &f, cudaStream_t s)
-{
-    k_bptt_dy<<<blocks_for(f.nb), kThreads, 0, s>>>(f.nodes, f.nb, f.a[0], f.y, f.scale, f.g, f.dy);
-    return cudaGetLastError();
-}
-
 cudaError_t bptt_scatter(const BpttFields &f, cudaStream_t s)
 {
     const Geo g{f.nx, f.ny, f.nz, f.nxp, f.sx, f.sy, f.sz};
-    k_bptt_feature_grad<<<blocks_for(f.nb), kThreads, 0, s>>>(f.nb, f.x, f.scale, f.kstar, f.g, f.y, f.dx);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
     k_bptt_gather<<<blocks_for(f.n_int), kThreads, 0, s>>>(g, f.n_int, f.sidx, f.dx, f.a[0], f.a[1], f.a[2]);
     return cudaGetLastError();
 }

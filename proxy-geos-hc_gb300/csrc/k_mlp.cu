@@ -1,31 +1,23 @@
-// k_mlp.cu -- kernels of the boundary network (mlp.h): BF16 tensor-core forward (mma.sync
-// m16n8k16, FP32 accumulators), the training pass (forward on the tensor cores, backward and
-// parameter gradients in FP32), Adam, and the boundary-strip gather / correction.
+// k_mlp.cu -- inference kernels of the boundary network (mlp.h): BF16 tensor-core forward (mma.sync
+// m16n8k16, FP32 accumulators) and the boundary-strip gather / correction.  Training and the
+// adjoint's network pass are in k_mlp_train.cu.
 //
 // Tile: 128 rows (samples or strip nodes) per CTA, 4 warps of 32 rows.  Shared memory holds the
 // BF16 weights as [out][in] rows (the MMA's column-major B operand) and the BF16 inputs and
 // hidden activations as row-major [row][in] (the row-major A operand); row strides are padded by
 // 8 elements so that the fragment loads of a warp hit 32 different banks.
-#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <vector>
 #include <cstddef>
 
-#include "mlp.h"
-#include "tma.cuh"
+#include "mlp_device.cuh"
 
 namespace semgb {
 
 namespace {
 
-// Fragment loads of the register-resident inference forward (compile-time knob: 1 = ldmatrix,
-// 0 = one 32-bit shared load per fragment register; the same fragments either way, so the same
-// bits).  ldmatrix: a quarter of the load instructions, 162 registers, no spill.
-#ifndef SEM_MLP_LDSM
-#define SEM_MLP_LDSM 1
-#endif
 // Face kernel staging (compile-time knob: 1 = the next tile's patch loads issued into registers
 // before the current tile's network runs, stored to shared memory after it; 0 = load and store
 // each tile's patch before its features).  The same values either way.
@@ -33,230 +25,13 @@ namespace {
 #define SEM_MLP_FACE_PIPE 1
 #endif
 
-constexpr int H = kMlpHidden;
-constexpr int KP1 = kMlpInPad + 8;  // row stride (bf16) of X and W1
-constexpr int KP2 = H + 8;          // row stride (bf16) of H1 and W2
-constexpr int T = kMlpTile;
-
-__device__ __forceinline__ uint16_t f2bf(float x)
-{
-    const __nv_bfloat16 b = __float2bfloat16_rn(x);
-    return *reinterpret_cast<const uint16_t *>(&b);
-}
-
-__device__ __forceinline__ float bf2f(uint16_t u)
-{
-    __nv_bfloat16 b;
-    *reinterpret_cast<uint16_t *>(&b) = u;
-    return __bfloat162float(b);
-}
-
-// two floats to BF16 (round to nearest even, as f2bf) in one conversion: lo in the low half
-__device__ __forceinline__ uint32_t pack_bf2(float lo, float hi)
-{
-    const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<const uint32_t *>(&b);
-}
-
-// GELU in the tanh form of Hendrycks & Gimpel (2016), GELU(z) = z/2 (1 + tanh(u)),
-// u = sqrt(2/pi) (z + 0.044715 z^3), and its derivative; tanh from the hardware approximation
-// (tanh.approx.f32, relative error about 2^-11, below the BF16 rounding of the activations)
-__device__ __forceinline__ float tanh_hw(float x)
-{
-    float y;
-    asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-constexpr float kGeluC = 0.7978845608028654f;  // sqrt(2/pi)
-constexpr float kGeluCA = 0.7978845608028654f * 0.044715f;
-// u = z (c + c a z^2): two multiplies and one fma
-__device__ __forceinline__ float gelu_u(float z) { return z * fmaf(kGeluCA, z * z, kGeluC); }
-__device__ __forceinline__ float gelu(float z)
-{
-    const float t = tanh_hw(gelu_u(z));
-    const float h = 0.5f * z;
-    return fmaf(h, t, h);
-}
-// gelu of two values with packed f32x2 arithmetic: the same operations in the same order as gelu,
-// each half rounded as the scalar instruction would round it
-__device__ __forceinline__ float2 gelu2(float2 z)
-{
-    const float2 w = fma2(make_float2(kGeluCA, kGeluCA), mul2(z, z), make_float2(kGeluC, kGeluC));
-    const float2 u = mul2(z, w);
-    const float2 t = make_float2(tanh_hw(u.x), tanh_hw(u.y));
-    const float2 h = mul2(make_float2(0.5f, 0.5f), z);
-    return fma2(h, t, h);
-}
-__device__ __forceinline__ float gelu_d(float z)
-{
-    // d/dz [z/2 (1 + tanh u)] = (1 + t)/2 + z/2 (1 - t^2) (c + 3 c a z^2)
-    const float t = tanh_hw(gelu_u(z));
-    return fmaf(0.5f, t, 0.5f) + (0.5f * z) * fmaf(-t, t, 1.f) * fmaf(3.f * kGeluCA, z * z, kGeluC);
-}
-
-__device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2])
-{
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-        "{%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
-
-#if SEM_MLP_LDSM
-// 8x8 b16 matrices from shared memory (fragment layout of the mma operands): x4 takes row
-// addresses from lanes 0-31 (matrix lane/8), x2 from lanes 0-15.
-__device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], const void *p)
-{
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p))));
-}
-__device__ __forceinline__ void ldsm_x2(uint32_t (&r)[2], const void *p)
-{
-    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0, %1}, [%2];"
-                 : "=r"(r[0]), "=r"(r[1])
-                 : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p))));
-}
-#endif
-
-struct NetSmem {
-    uint16_t w1[H * KP1];
-    uint16_t w2[H * KP2];
-    float b1[H], b2[H], w3[H], b3;
-};
-
-__device__ void load_net(NetSmem &s, const MlpDev &net)
-{
-    // 16-byte chunks: W1 rows are 96 bf16 (12 chunks), W2 rows 64 (8 chunks); shared rows are
-    // padded to 104 and 72 elements, still 16-byte aligned
-    constexpr int C1 = kMlpInPad / 8, C2 = H / 8;
-    static_assert((KP1 * 2) % 16 == 0 && (KP2 * 2) % 16 == 0, "16-byte aligned shared rows");
-#pragma unroll 4
-    for (int i = threadIdx.x; i < H * C1; i += blockDim.x) {
-        const int nn = i / C1, j = i - nn * C1;
-        *reinterpret_cast<uint4 *>(s.w1 + nn * KP1 + j * 8) = __ldg(reinterpret_cast<const uint4 *>(net.w1) + i);
-    }
-#pragma unroll 4
-    for (int i = threadIdx.x; i < H * C2; i += blockDim.x) {
-        const int nn = i / C2, j = i - nn * C2;
-        *reinterpret_cast<uint4 *>(s.w2 + nn * KP2 + j * 8) = __ldg(reinterpret_cast<const uint4 *>(net.w2) + i);
-    }
-    for (int i = threadIdx.x; i < H; i += blockDim.x) {
-        s.b1[i] = net.b1[i];
-        s.b2[i] = net.b2[i];
-        s.w3[i] = net.w3[i];
-    }
-    if (threadIdx.x == 0) s.b3 = net.b3[0];
-}
-
-// Forward of the warp's 32 rows (tile rows wr..wr+31): xs [T][KP1] bf16 in, h1 [T][KP2] bf16
-// written, returns y for rows wr + mt*16 + g (+8) in yv[mt][0/1] (valid on every lane of a quad).
-// With z1/z2 non-null the pre-activations are kept (FP32 [T][H]).
-__device__ void forward_rows(const NetSmem &s, const uint16_t *xs, uint16_t *h1, float *z1, float *z2, int wr,
-                             float (&yv)[2][2])
-{
-    const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-    float acc[2][8][4];
-#pragma unroll
-    for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-        for (int nt = 0; nt < 8; nt++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) acc[mt][nt][j] = 0.f;
-#pragma unroll
-    for (int ks = 0; ks < kMlpInPad / 16; ks++) {
-        const int k0 = ks * 16 + q * 2;
-        uint32_t a[2][4];
-#pragma unroll
-        for (int mt = 0; mt < 2; mt++) {
-            const int r = wr + mt * 16 + g;
-            a[mt][0] = *reinterpret_cast<const uint32_t *>(xs + r * KP1 + k0);
-            a[mt][1] = *reinterpret_cast<const uint32_t *>(xs + (r + 8) * KP1 + k0);
-            a[mt][2] = *reinterpret_cast<const uint32_t *>(xs + r * KP1 + k0 + 8);
-            a[mt][3] = *reinterpret_cast<const uint32_t *>(xs + (r + 8) * KP1 + k0 + 8);
-        }
-#pragma unroll
-        for (int nt = 0; nt < 8; nt++) {
-            const int n = nt * 8 + g;
-            uint32_t b[2];
-            b[0] = *reinterpret_cast<const uint32_t *>(s.w1 + n * KP1 + k0);
-            b[1] = *reinterpret_cast<const uint32_t *>(s.w1 + n * KP1 + k0 + 8);
-            mma16816(acc[0][nt], a[0], b);
-            mma16816(acc[1][nt], a[1], b);
-        }
-    }
-    // layer-1 epilogue: bias, GELU, BF16 into h1 (the warp's own rows)
-#pragma unroll
-    for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-        for (int nt = 0; nt < 8; nt++) {
-            const int c = nt * 8 + q * 2;
-#pragma unroll
-            for (int hrow = 0; hrow < 2; hrow++) {
-                const int r = wr + mt * 16 + g + hrow * 8;
-                const float za = acc[mt][nt][hrow * 2] + s.b1[c], zb = acc[mt][nt][hrow * 2 + 1] + s.b1[c + 1];
-                if (z1) {
-                    z1[r * H + c] = za;
-                    z1[r * H + c + 1] = zb;
-                }
-                *reinterpret_cast<uint32_t *>(h1 + r * KP2 + c) = pack_bf2(gelu(za), gelu(zb));
-                acc[mt][nt][hrow * 2] = 0.f;
-                acc[mt][nt][hrow * 2 + 1] = 0.f;
-            }
-        }
-    __syncwarp();
-#pragma unroll
-    for (int ks = 0; ks < H / 16; ks++) {
-        const int k0 = ks * 16 + q * 2;
-        uint32_t a[2][4];
-#pragma unroll
-        for (int mt = 0; mt < 2; mt++) {
-            const int r = wr + mt * 16 + g;
-            a[mt][0] = *reinterpret_cast<const uint32_t *>(h1 + r * KP2 + k0);
-            a[mt][1] = *reinterpret_cast<const uint32_t *>(h1 + (r + 8) * KP2 + k0);
-            a[mt][2] = *reinterpret_cast<const uint32_t *>(h1 + r * KP2 + k0 + 8);
-            a[mt][3] = *reinterpret_cast<const uint32_t *>(h1 + (r + 8) * KP2 + k0 + 8);
-        }
-#pragma unroll
-        for (int nt = 0; nt < 8; nt++) {
-            const int n = nt * 8 + g;
-            uint32_t b[2];
-            b[0] = *reinterpret_cast<const uint32_t *>(s.w2 + n * KP2 + k0);
-            b[1] = *reinterpret_cast<const uint32_t *>(s.w2 + n * KP2 + k0 + 8);
-            mma16816(acc[0][nt], a[0], b);
-            mma16816(acc[1][nt], a[1], b);
-        }
-    }
-    // layer-2 epilogue and the output layer: y = b3 + sum_c w3[c] GELU(z2[c])
-#pragma unroll
-    for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-        for (int hrow = 0; hrow < 2; hrow++) {
-            const int r = wr + mt * 16 + g + hrow * 8;
-            float part = 0.f;
-#pragma unroll
-            for (int nt = 0; nt < 8; nt++) {
-                const int c = nt * 8 + q * 2;
-                const float za = acc[mt][nt][hrow * 2] + s.b2[c], zb = acc[mt][nt][hrow * 2 + 1] + s.b2[c + 1];
-                if (z2) {
-                    z2[r * H + c] = za;
-                    z2[r * H + c + 1] = zb;
-                }
-                part = fmaf(s.w3[c], gelu(za), part);
-                part = fmaf(s.w3[c + 1], gelu(zb), part);
-            }
-            part += __shfl_xor_sync(0xffffffffu, part, 1);
-            part += __shfl_xor_sync(0xffffffffu, part, 2);
-            yv[mt][hrow] = part + s.b3;
-        }
-}
-
-// As forward_rows for inference (no saved activations), with the hidden layer kept in registers:
+// Forward of the warp's 32 rows (tile rows wr..wr+31): xs [T][KP1] bf16 in, y for rows
+// wr + mt*16 + g (+8) in yv[mt][0/1] (valid on every lane of a quad).  The hidden layer stays in
+// registers:
 // the m16n8 accumulator fragments of layer-1 columns 16k..16k+15 (n-tiles 2k and 2k+1) are, after
 // bias, GELU and BF16 rounding, exactly the m16n8k16 A fragments of layer 2's k-step k, so no
 // shared-memory copy of the hidden activations is made.  Same roundings and summation order as
-// forward_rows, which the training and the adjoint use: a network must be trained and
+// the training forward (k_mlp_train.cu): a network must be trained and
 // differentiated as it runs, and the training of the learned boundary, a feedback loop over whole
 // runs, follows last-bit differences far (biases entered as the first MMA's accumulator, which
 // round the pre-activations differently, moved the reflected energy of the network trained with
@@ -368,6 +143,11 @@ __device__ void forward_rows_regs(const NetSmem &s, const uint16_t *xs, int wr, 
         }
 }
 
+static_assert(offsetof(NetSmem, b1) % 8 == 0 && offsetof(NetSmem, b2) % 8 == 0, "bias pairs load as float2");
+// features start on a 16-byte boundary after the weights (their rows are stored 16 bytes at a time)
+constexpr size_t kAbcXsOff = (sizeof(NetSmem) + 15) / 16 * 16;
+static_assert((KP1 * sizeof(uint16_t)) % 16 == 0 && kMlpInPad % 8 == 0, "16-byte feature rows");
+
 // stage rows [row0, row0 + T) of x [n][81] (FP32, scaled by 1/scale[i] when scale is given) as
 // BF16 [T][KP1] with zero padding
 __device__ void stage_x(uint16_t *xs, const float *x, int64_t row0, int64_t n)
@@ -384,8 +164,7 @@ __global__ void __launch_bounds__(128) k_mlp_forward(const MlpDev net, const flo
 {
     extern __shared__ __align__(16) unsigned char smem[];
     NetSmem &s = *reinterpret_cast<NetSmem *>(smem);
-    uint16_t *xs = reinterpret_cast<uint16_t *>(smem + sizeof(NetSmem));
-    uint16_t *h1 = xs + T * KP1;
+    uint16_t *xs = reinterpret_cast<uint16_t *>(smem + kAbcXsOff);
     load_net(s, net);
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
     for (int64_t row0 = (int64_t)blockIdx.x * T; row0 < n; row0 += (int64_t)gridDim.x * T) {
@@ -393,7 +172,7 @@ __global__ void __launch_bounds__(128) k_mlp_forward(const MlpDev net, const flo
         stage_x(xs, x, row0, n);
         __syncthreads();
         float yv[2][2];
-        forward_rows(s, xs, h1, nullptr, nullptr, w * 32, yv);
+        forward_rows_regs(s, xs, w * 32, yv);
         if (q == 0)
 #pragma unroll
             for (int mt = 0; mt < 2; mt++)
@@ -405,239 +184,12 @@ __global__ void __launch_bounds__(128) k_mlp_forward(const MlpDev net, const flo
     }
 }
 
-// Training pass: loss and parameter gradients over all n samples, accumulated per CTA in shared
-// memory (each gradient entry owned by one thread) and added to the global buffers once.
-struct TrainSmem {
-    float z1[T * H];
-    float z2[T * H];
-    float dy[T];
-    float g[kMlpParams];
-};
-
-// dy_in non-null: the gradient of the output per row is given (dy_in[row]; no loss), otherwise
-// dy = 2 (y - t) / n.  dx_out non-null: the gradient with respect to the (BF16-rounded) inputs,
-// dx[row][k] = sum_n dZ1[row][n] W1[n][k] (k < 81), is written too.
-__global__ void __launch_bounds__(128) k_mlp_train_pass(const MlpDev net, const float *x, const float *t, int64_t n,
-                                                        double *part_loss, float *part, const float *dy_in,
-                                                        float *dx_out)
-{
-    extern __shared__ __align__(16) unsigned char smem[];
-    NetSmem &s = *reinterpret_cast<NetSmem *>(smem);
-    uint16_t *xs = reinterpret_cast<uint16_t *>(smem + sizeof(NetSmem));
-    uint16_t *h1 = xs + T * KP1;
-    TrainSmem &ts = *reinterpret_cast<TrainSmem *>(h1 + T * KP2);
-    load_net(s, net);
-    for (int i = threadIdx.x; i < kMlpParams; i += blockDim.x) ts.g[i] = 0.f;
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-    const int tid = threadIdx.x;
-    const float inv_n = 1.f / (float)n;
-    double lsum = 0.0;
-    for (int64_t row0 = (int64_t)blockIdx.x * T; row0 < n; row0 += (int64_t)gridDim.x * T) {
-        __syncthreads();
-        stage_x(xs, x, row0, n);
-        __syncthreads();
-        float yv[2][2];
-        forward_rows(s, xs, h1, ts.z1, ts.z2, w * 32, yv);
-        if (q == 0)
-#pragma unroll
-            for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-                for (int hrow = 0; hrow < 2; hrow++) {
-                    const int r = w * 32 + mt * 16 + g + hrow * 8;
-                    const int64_t row = row0 + r;
-                    float d = 0.f;
-                    if (row < n) {
-                        if (dy_in) {
-                            d = dy_in[row];
-                        } else {
-                            const float e = yv[mt][hrow] - t[row];
-                            lsum += (double)e * e;
-                            d = 2.f * e * inv_n;
-                        }
-                    }
-                    ts.dy[r] = d;
-                }
-        __syncthreads();
-        // row pass (thread = row): output layer, dZ2 = dy w3 GELU'(z2) in place of z2
-        {
-            const int r = tid;
-            const float d = ts.dy[r];
-            for (int c = 0; c < H; c++) {
-                const float z = ts.z2[r * H + c];
-                ts.z2[r * H + c] = d * s.w3[c] * gelu_d(z);
-            }
-        }
-        __syncthreads();
-        // column sums: db2[c] (thread c < 64) and db3; dw3 needs GELU(z2), which this pass
-        // overwrites, so k_mlp_grad_w3 accumulates it from a second forward
-        if (tid < H) {
-            float a2 = 0.f;
-            for (int r = 0; r < T; r++) a2 += ts.z2[r * H + tid];
-            ts.g[kOffB2 + tid] += a2;
-        } else if (tid == H) {
-            float a = 0.f;
-            for (int r = 0; r < T; r++) a += ts.dy[r];
-            ts.g[kOffB3] += a;
-        }
-        // dW2[n][k] = sum_r dZ2[r][n] H1[r][k]: 4096 entries, 32 per thread
-        for (int e = tid; e < H * H; e += blockDim.x) {
-            const int nn = e / H, k = e - nn * H;
-            float a = 0.f;
-            for (int r = 0; r < T; r++) a = fmaf(ts.z2[r * H + nn], bf2f(h1[r * KP2 + k]), a);
-            ts.g[kOffW2 + e] += a;
-        }
-        __syncthreads();
-        // row pass: dZ1[r][k] = GELU'(z1[r][k]) sum_n dZ2[r][n] W2[n][k], in place of z1
-        {
-            const int r = tid;
-            float dh[H];
-#pragma unroll
-            for (int k = 0; k < H; k++) dh[k] = 0.f;
-            for (int nn = 0; nn < H; nn++) {
-                const float dz = ts.z2[r * H + nn];
-#pragma unroll
-                for (int k = 0; k < H; k++) dh[k] = fmaf(dz, bf2f(s.w2[nn * KP2 + k]), dh[k]);
-            }
-#pragma unroll
-            for (int k = 0; k < H; k++) ts.z1[r * H + k] = dh[k] * gelu_d(ts.z1[r * H + k]);
-            if (dx_out && row0 + r < n) {
-                // input gradient of the row from its own dZ1 (this thread's row only)
-                float *dxr = dx_out + (row0 + r) * kMlpIn;
-                for (int k = 0; k < kMlpIn; k++) {
-                    float a = 0.f;
-                    for (int nn = 0; nn < H; nn++) a = fmaf(ts.z1[r * H + nn], bf2f(s.w1[nn * KP1 + k]), a);
-                    dxr[k] = a;
-                }
-            }
-        }
-        __syncthreads();
-        // db1 and dW1[n][k] = sum_r dZ1[r][n] X[r][k] (k < 81)
-        if (tid < H) {
-            float a = 0.f;
-            for (int r = 0; r < T; r++) a += ts.z1[r * H + tid];
-            ts.g[kOffB1 + tid] += a;
-        }
-        for (int e = tid; e < H * kMlpIn; e += blockDim.x) {
-            const int nn = e / kMlpIn, k = e - nn * kMlpIn;
-            float a = 0.f;
-            for (int r = 0; r < T; r++) a = fmaf(ts.z1[r * H + nn], bf2f(xs[r * KP1 + k]), a);
-            ts.g[kOffW1 + e] += a;
-        }
-        __syncthreads();
-    }
-    __syncthreads();
-    // this CTA's partial sums (the W3 range is written by k_mlp_grad_w3)
-    float *pg = part + (int64_t)blockIdx.x * kMlpParams;
-    for (int i = threadIdx.x; i < kMlpParams; i += blockDim.x)
-        if (i < kOffW3 || i >= kOffW3 + H) pg[i] = ts.g[i];
-    // loss: quad leaders hold partial sums; warps added in order
-    lsum += __shfl_xor_sync(0xffffffffu, lsum, 4);
-    lsum += __shfl_xor_sync(0xffffffffu, lsum, 8);
-    lsum += __shfl_xor_sync(0xffffffffu, lsum, 16);
-    __shared__ double wl[4];
-    if (lane == 0) wl[w] = lsum;
-    __syncthreads();
-    if (threadIdx.x == 0) part_loss[blockIdx.x] = (((wl[0] + wl[1]) + wl[2]) + wl[3]) / (double)n;
-}
-
-// grad[i] += sum over CTAs b (in order) of part[b][i]; *loss += sum of part_loss[b] in order
-__global__ void k_mlp_reduce(const float *part, const double *part_loss, int nb, float *grad, double *loss)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < kMlpParams) {
-        float a = 0.f;
-        for (int b = 0; b < nb; b++) a += part[(int64_t)b * kMlpParams + i];
-        grad[i] += a;
-    }
-    if (i == 0) {
-        double l = 0.0;
-        for (int b = 0; b < nb; b++) l += part_loss[b];
-        *loss += l;
-    }
-}
-
-// dw3[c] = sum_r dy[r] GELU(z2[r][c]) needs the forward activations the training pass
-// overwrites; this pass recomputes them (forward only) and accumulates dw3.
-__global__ void __launch_bounds__(128) k_mlp_grad_w3(const MlpDev net, const float *x, const float *t, int64_t n,
-                                                     float *part, const float *dy_in)
-{
-    extern __shared__ __align__(16) unsigned char smem[];
-    NetSmem &s = *reinterpret_cast<NetSmem *>(smem);
-    uint16_t *xs = reinterpret_cast<uint16_t *>(smem + sizeof(NetSmem));
-    uint16_t *h1 = xs + T * KP1;
-    float *z2 = reinterpret_cast<float *>(h1 + T * KP2);
-    float *dy = z2 + T * H;
-    float *gw3 = dy + T;
-    load_net(s, net);
-    for (int i = threadIdx.x; i < H; i += blockDim.x) gw3[i] = 0.f;
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-    const float inv_n = 1.f / (float)n;
-    for (int64_t row0 = (int64_t)blockIdx.x * T; row0 < n; row0 += (int64_t)gridDim.x * T) {
-        __syncthreads();
-        stage_x(xs, x, row0, n);
-        __syncthreads();
-        float yv[2][2];
-        forward_rows(s, xs, h1, nullptr, z2, w * 32, yv);
-        if (q == 0)
-#pragma unroll
-            for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-                for (int hrow = 0; hrow < 2; hrow++) {
-                    const int r = w * 32 + mt * 16 + g + hrow * 8;
-                    const int64_t row = row0 + r;
-                    dy[r] = row < n ? (dy_in ? dy_in[row] : 2.f * (yv[mt][hrow] - t[row]) * inv_n) : 0.f;
-                }
-        __syncthreads();
-        if (threadIdx.x < H) {
-            const int c = threadIdx.x;
-            float a = 0.f;
-            for (int r = 0; r < T; r++) a = fmaf(dy[r], gelu(z2[r * H + c]), a);
-            gw3[c] += a;
-        }
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < H; i += blockDim.x) part[(int64_t)blockIdx.x * kMlpParams + kOffW3 + i] = gw3[i];
-}
-
-__global__ void k_mlp_pack(const float *m, uint16_t *w1, uint16_t *w2, float *b1, float *b2, float *w3, float *b3)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < H * kMlpInPad) {
-        const int nn = i / kMlpInPad, k = i - nn * kMlpInPad;
-        w1[i] = f2bf(k < kMlpIn ? m[kOffW1 + nn * kMlpIn + k] : 0.f);
-    }
-    if (i < H * H) w2[i] = f2bf(m[kOffW2 + i]);
-    if (i < H) {
-        b1[i] = m[kOffB1 + i];
-        b2[i] = m[kOffB2 + i];
-        w3[i] = m[kOffW3 + i];
-    }
-    if (i == 0) b3[0] = m[kOffB3];
-}
-
-__global__ void k_mlp_adam(float *p, const float *g, float *m, float *v, float lr, float c1, float c2)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= kMlpParams) return;
-    const float gi = g[i];
-    const float mi = 0.9f * m[i] + 0.1f * gi;
-    const float vi = 0.999f * v[i] + 0.001f * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    p[i] -= lr * (mi * c1) / (sqrtf(vi * c2) + 1e-8f);
-}
-
 // ---- boundary strip ---------------------------------------------------------------------------
 
 // Four CTAs per SM: the weights, the features and the scales fit 4 x 51 KB of shared memory,
 // the hidden layer stays in registers (forward_rows_regs).  Warp w gathers rows 32w..32w+31 of
 // the tile and runs the network on the same rows, so after the weights are staged the warps
 // only synchronise with themselves.
-static_assert(offsetof(NetSmem, b1) % 8 == 0 && offsetof(NetSmem, b2) % 8 == 0, "bias pairs load as float2");
-// features start on a 16-byte boundary after the weights (their rows are stored 16 bytes at a time)
-constexpr size_t kAbcXsOff = (sizeof(NetSmem) + 15) / 16 * 16;
-static_assert((KP1 * sizeof(uint16_t)) % 16 == 0 && kMlpInPad % 8 == 0, "16-byte feature rows");
-
 __global__ void __launch_bounds__(128, 4) k_abc_correction(const MlpDev net, const AbcArgs a)
 {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -963,20 +515,7 @@ __global__ void k_abc_history(const int64_t *shell, int64_t n, const float *p_cu
     }
 }
 
-__global__ void k_gather_rows(const float *x, const float *t, const int64_t *idx, int64_t nb, float *bx, float *bt)
-{
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nb * kMlpIn;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = i / kMlpIn, k = i - r * kMlpIn;
-        const int64_t src = idx[r];
-        bx[i] = x[src * kMlpIn + k];
-        if (k == 0) bt[r] = t[src];
-    }
-}
-
-size_t smem_forward() { return sizeof(NetSmem) + sizeof(uint16_t) * T * (KP1 + KP2); }
-size_t smem_train() { return smem_forward() + sizeof(TrainSmem); }
-size_t smem_w3() { return smem_forward() + sizeof(float) * (T * H + T + H); }
+size_t smem_forward() { return kAbcXsOff + sizeof(uint16_t) * T * KP1; }
 size_t smem_abc() { return kAbcXsOff + sizeof(uint16_t) * T * KP1 + sizeof(float) * T; }
 size_t smem_face() { return kFaceOffsOff + sizeof(int) * 32; }
 
@@ -988,13 +527,6 @@ int grid_for(int64_t n)
 
 }  // namespace
 
-cudaError_t mlp_pack(const float *master, uint16_t *w1, uint16_t *w2, float *b1, float *b2, float *w3, float *b3,
-                     cudaStream_t s)
-{
-    k_mlp_pack<<<(H * kMlpInPad + 255) / 256, 256, 0, s>>>(master, w1, w2, b1, b2, w3, b3);
-    return cudaGetLastError();
-}
-
 cudaError_t mlp_forward(const MlpDev &net, const float *x, float *y, int64_t n, cudaStream_t s)
 {
     if (n <= 0) return cudaSuccess;
@@ -1002,41 +534,6 @@ cudaError_t mlp_forward(const MlpDev &net, const float *x, float *y, int64_t n, 
     cudaError_t e = cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
     k_mlp_forward<<<grid_for(n), T, sm, s>>>(net, x, y, n);
-    return cudaGetLastError();
-}
-
-cudaError_t mlp_loss_grad(const MlpDev &net, const float *x, const float *t, int64_t n, double *loss, float *grad,
-                          float *part, double *part_loss, cudaStream_t s, const float *dy_in, float *dx_out)
-{
-    if (n <= 0) return cudaSuccess;
-    const int nb = grid_for(n);
-    static_assert(kMlpMaxCTAs >= 152 * 4, "partial-sum rows for every CTA of grid_for");
-    size_t sm = smem_train();
-    cudaError_t e = cudaFuncSetAttribute(k_mlp_train_pass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    k_mlp_train_pass<<<nb, T, sm, s>>>(net, x, t, n, part_loss, part, dy_in, dx_out);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    sm = smem_w3();
-    if ((e = cudaFuncSetAttribute(k_mlp_grad_w3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) != cudaSuccess)
-        return e;
-    k_mlp_grad_w3<<<nb, T, sm, s>>>(net, x, t, n, part, dy_in);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    k_mlp_reduce<<<(kMlpParams + 255) / 256, 256, 0, s>>>(part, part_loss, nb, grad, loss);
-    return cudaGetLastError();
-}
-
-cudaError_t mlp_adam(float *master, const float *grad, float *m, float *v, int t, float lr, cudaStream_t s)
-{
-    const float c1 = 1.f / (1.f - powf(0.9f, (float)t)), c2 = 1.f / (1.f - powf(0.999f, (float)t));
-    k_mlp_adam<<<(kMlpParams + 255) / 256, 256, 0, s>>>(master, grad, m, v, lr, c1, c2);
-    return cudaGetLastError();
-}
-
-cudaError_t mlp_gather_rows(const float *x, const float *t, const int64_t *idx, int64_t nb, float *bx, float *bt,
-                            cudaStream_t s)
-{
-    if (nb > 0)
-        k_gather_rows<<<(int)std::min<int64_t>((nb * kMlpIn + 255) / 256, 152 * 16), 256, 0, s>>>(x, t, idx, nb, bx, bt);
     return cudaGetLastError();
 }
 

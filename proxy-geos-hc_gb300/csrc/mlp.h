@@ -81,11 +81,7 @@ struct BpttFields {
     const int64_t *nodes;       // boundary nodes (device layout), nb of them
     int64_t nb;
     const int *sidx;            // [n_int]: index in `nodes`, -1 elsewhere
-    float *x;                   // [nb][81] features divided by the scale
-    float *scale;               // [nb]
-    int *kstar;                 // [nb] arg-max feature | 0x100 if negative; -1: all zero
-    float *y, *g, *dy;          // [nb] network output, adjoint of the node's new value, output gradient
-    float *dx;                  // [nb][81] input gradient, then feature gradient
+    float *dx;                  // [nb][81] feature gradient
     float *a[3];                // adjoints of out^m, out^{m-1}, out^{m-2}
     float *v;                   // [n_int] work field
     const int64_t *roi;         // region of interest (device layout), n_roi nodes
@@ -99,11 +95,7 @@ struct BpttOperator {
     float wa[kMaxOrder];
     float g[3];
 };
-// Features of the boundary nodes from out^m, out^{m-1}, out^{m-2}.
-cudaError_t bptt_features(const BpttFields &f, const float *lm, const float *lm1, const float *lm2, cudaStream_t s);
-// g and dy from A0 and the network output y.
-cudaError_t bptt_dy(const BpttFields &f, cudaStream_t s);
-// dx -> feature gradient, gathered into A0, A1, A2.
+// Feature gradients gathered into A0, A1, A2.
 cudaError_t bptt_scatter(const BpttFields &f, cudaStream_t s);
 // Interior leapfrog adjoint (A0 -> A1, A2); a_mass = dt^2 / M.
 cudaError_t bptt_interior(const BpttFields &f, const BpttOperator &op, const float *a_mass, cudaStream_t s);
@@ -115,22 +107,47 @@ cudaError_t mlp_pack(const float *master, uint16_t *w1, uint16_t *w2, float *b1,
                      cudaStream_t s);
 // y[i] = net(x[i]) for x [n][81] (FP32, device).
 cudaError_t mlp_forward(const MlpDev &net, const float *x, float *y, int64_t n, cudaStream_t s);
+// Work arrays of a training pass (k_mlp_train.cu), rows of one round (mlp_work_rows).
+constexpr int kMlpMaxSlots = 152 * 4;  // partial-sum slots: tile t of a pass adds to slot t % kMlpMaxSlots
+constexpr int kMlpXbStride = 88;       // row stride (bf16) of the stored inputs
+struct MlpWork {
+    uint16_t *xb = nullptr;   // [rows][88] BF16 inputs
+    uint16_t *h1 = nullptr;   // [rows][64] BF16 hidden activations
+    float *dz1 = nullptr, *dz2 = nullptr, *g2 = nullptr;  // [rows][64] dZ of both layers, GELU(z2)
+    float *err = nullptr, *dy = nullptr;                  // [rows] y - t, output gradient
+    float *part = nullptr;    // [kMlpMaxSlots][kMlpParams] partial gradients
+    double *lsum = nullptr;   // [kMlpMaxSlots][32] partial squared errors
+};
+// Rows of work arrays that a pass over n rows needs (at most kMlpMaxSlots tiles: longer passes run
+// in rounds).
+int64_t mlp_work_rows(int64_t n);
+// Adam on the FP32 master parameters: moments, step count (from 1) and rate, and the kernels' form
+// of the network, rewritten with the new parameters.
+struct MlpAdam {
+    float *master, *m, *v;
+    int t;
+    float lr;
+    uint16_t *w1, *w2;
+    float *b1, *b2, *w3, *b3;
+};
+// Shared-memory limits of the training kernels on the current device.
+cudaError_t mlp_train_setup();
 // Loss 1/n sum (net(x_i) - t_i)^2 accumulated into *loss (double), gradients with respect to the
-// master parameters accumulated into grad (FP32 [kMlpParams]).
-// Deterministic: every CTA writes its partial sums to part ([kMlpMaxCTAs][kMlpParams]) and
-// part_loss ([kMlpMaxCTAs]), and one pass adds them in CTA order.
-constexpr int kMlpMaxCTAs = 152 * 4;
-// With dy_in (device, [n]) the output gradient per row is given instead of the squared-error loss
-// (t is not read and the loss is not accumulated); with dx_out (device, [n][81]) the gradient with
-// respect to the inputs is written too.
+// master parameters accumulated into grad (FP32 [kMlpParams]).  Deterministic: partial sums per
+// tile, added in order.
 cudaError_t mlp_loss_grad(const MlpDev &net, const float *x, const float *t, int64_t n, double *loss, float *grad,
-                          float *part, double *part_loss, cudaStream_t s, const float *dy_in = nullptr,
-                          float *dx_out = nullptr);
-// bx[i] = x[idx[i]], bt[i] = t[idx[i]] for i < nb (minibatch rows).
-cudaError_t mlp_gather_rows(const float *x, const float *t, const int64_t *idx, int64_t nb, float *bx, float *bt,
-                            cudaStream_t s);
-// Adam step on the FP32 master weights (m, v moments; t = step count starting at 1).
-cudaError_t mlp_adam(float *master, const float *grad, float *m, float *v, int t, float lr, cudaStream_t s);
+                          const MlpWork &w, cudaStream_t s);
+// One minibatch of Adam on samples idx[0..n): the loss before the step into *loss.  dependent: the
+// preceding work of the stream is a step on the same network.
+cudaError_t mlp_train_step(const MlpDev &net, const float *x, const float *t, const int64_t *idx, int64_t n,
+                           double *loss, const MlpAdam &adam, const MlpWork &w, cudaStream_t s, bool dependent);
+// One step of the adjoint of the time loop at the boundary nodes: features from the levels out^m,
+// out^{m-1}, out^{m-2}, output gradient from A0, parameter gradients added to grad, feature
+// gradients into f.dx.
+cudaError_t mlp_boundary_grad(const MlpDev &net, const BpttFields &f, const float *lm, const float *lm1,
+                              const float *lm2, float *grad, const MlpWork &w, cudaStream_t s);
+// One Adam step with a given gradient.
+cudaError_t mlp_adam(const MlpAdam &adam, const float *grad, cudaStream_t s);
 // Boundary correction: corr[i] = scale_i * net(features_i / scale_i) for the strip nodes.
 cudaError_t abc_correction(const MlpDev &net, const AbcArgs &a, cudaStream_t s);
 // p_new[node_i] += corr[i].

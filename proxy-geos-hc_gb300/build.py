@@ -21,7 +21,7 @@ LIB = os.path.join(OUT_DIR, "libsemgb.so")
 
 SOURCES = ["api.cu", "adjoint_api.cu", "batch_api.cu", "group_api.cu", "k_group.cu", "k_bptt.cu", "abc_api.cu", "k_mlp.cu", "k_mlp_train.cu", "k_element.cu", "k_update.cu", "k_stencil.cu", "k_batch.cu", "noalloc.cu",
            "host_util.cpp", "formats.cpp"]
-HEADERS = ["abi.h", "stencil_body.cuh", "solver.h", "batch.h", "mlp.h", "mlp_device.cuh", "kernels.h", "stencil.h", "host_util.h", "tma.cuh"]
+HEADERS = ["abi.h", "stencil_body.cuh", "solver.h", "batch.h", "mlp.h", "mlp_device.cuh", "launch.cuh", "kernels.h", "stencil.h", "host_util.h", "tma.cuh"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 

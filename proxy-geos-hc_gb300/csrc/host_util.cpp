@@ -1,6 +1,7 @@
 // host_util.cpp -- GLL tables, Ricker wavelet, box indexing and sponge profile (host side).
 #include "host_util.h"
 
+#include <array>
 #include <cmath>
 
 namespace semgb {
@@ -22,9 +23,8 @@ void legendre(int n, double x, double &p, double &dp)
 
 }  // namespace
 
-bool gll_tables(int order, Gll &g)
+static void compute_gll_tables(int order, Gll &g)
 {
-    if (order < kMinOrder || order > kMaxOrder) return false;
     const int N = order, n1 = order + 1;
     g.order = order;
     g.xi[0] = -1.0;
@@ -65,6 +65,19 @@ bool gll_tables(int order, Gll &g)
             else d = 0.0;
             g.dphi[j * n1 + i] = d;
         }
+}
+
+bool gll_tables(int order, Gll &g)
+{
+    if (order < kMinOrder || order > kMaxOrder) return false;
+    // computed once per process (the Newton iterations take tens of microseconds, which the
+    // allocation-free step would otherwise pay on every call)
+    static const std::array<Gll, kMaxOrder + 1> tables = [] {
+        std::array<Gll, kMaxOrder + 1> t{};
+        for (int o = kMinOrder; o <= kMaxOrder; o++) compute_gll_tables(o, t[o]);
+        return t;
+    }();
+    g = tables[order];
     return true;
 }
 

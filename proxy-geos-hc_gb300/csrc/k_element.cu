@@ -26,8 +26,10 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "kernels.h"
+#include "launch.cuh"
 
 namespace semgb {
 
@@ -144,12 +146,31 @@ __global__ void __launch_bounds__(ElemCfg<O>::THREADS, ElemCfg<O>::MINB)
 #pragma unroll
         for (int i = 0; i < O1; i++) {
             const int g = cr[i + O1 * jx + NP * kx];
-            v[i] = act && (!CHECKED || (g >= 0 && g < a.n_check)) ? __ldg(a.p + g) : 0.f;
+            // (CHECKED: an ordinary load, which is not moved above the wait for the preceding launch)
+            if constexpr (CHECKED) v[i] = act && g >= 0 && g < a.n_check ? a.p[g] : 0.f;
+            else v[i] = act ? __ldg(a.p + g) : 0.f;
         }
     };
 
     // A: coefficient table, the first two tiles' rows, and the first tile's pencil values
-    for (int q = tid; q < C::TAB; q += C::THREADS) s_tab[q] = __ldg((REF ? a.rtab : a.tab) + q);
+    if constexpr (CHECKED) {
+        for (int q = tid; q < 3 * NP; q += C::THREADS) {
+            const int d = q / NP, r = q - d * NP, i = r % O1, j = r / O1;
+            float wi = 0.f, wj = 0.f;
+#pragma unroll
+            for (int k = 0; k < O1; k++) {  // static indices keep the parameter arrays out of local memory
+                if (k == i) wi = a.w[k];
+                if (k == j) wj = a.w[k];
+            }
+            s_tab[q] = (d == 0 ? a.g[0] : (d == 1 ? a.g[1] : a.g[2])) * wi * wj;
+        }
+        // launched behind the update of the step before (launch_after): nothing of the caller's is
+        // read, and the accumulator not added to, before that has finished
+        grid_dependency_wait();
+        grid_launch_dependents();
+    } else {
+        for (int q = tid; q < C::TAB; q += C::THREADS) s_tab[q] = __ldg((REF ? a.rtab : a.tab) + q);
+    }
     load_conn(t, 0);
     load_conn(t + gridDim.x, 1);
     cp_async_wait_one();
@@ -278,18 +299,15 @@ cudaError_t launch_element_r(const ElementArgs &a, cudaStream_t s)
     using C = ElemCfg<O, REF>;
     if (a.n_elem <= 0) return cudaSuccess;
     const int64_t tiles = (a.n_elem + C::TE - 1) / C::TE;
-    // persistent CTAs: as many as are resident at once
-    int dev = 0, sms = 152, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_element<O, REF, CHECKED>, C::THREADS, C::SMEM) !=
-            cudaSuccess ||
-        per_sm < 1) {
-        cudaGetLastError();
-        per_sm = 1;
-    }
-    const int64_t grid = std::min<int64_t>(tiles, (int64_t)sms * per_sm);
-    k_element<O, REF, CHECKED><<<(unsigned)grid, C::THREADS, C::SMEM, s>>>(a);
+    // persistent CTAs: as many as are resident at once (looked up once per device: the occupancy
+    // query costs the host microseconds on every step)
+    static std::atomic<int> resident[kMaxLaunchDevices];
+    int n = 0;
+    cudaError_t e = resident_ctas(k_element<O, REF, CHECKED>, C::THREADS, C::SMEM, resident, n);
+    if (e != cudaSuccess) return e;
+    const unsigned grid = (unsigned)std::min<int64_t>(tiles, n);
+    if constexpr (CHECKED) return launch_after(k_element<O, REF, CHECKED>, dim3(grid), C::THREADS, C::SMEM, s, true, a);
+    k_element<O, REF, CHECKED><<<grid, C::THREADS, C::SMEM, s>>>(a);
     return cudaGetLastError();
 }
 

@@ -29,6 +29,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "launch.cuh"
 #include "mlp_device.cuh"
 
 namespace semgb {
@@ -38,11 +39,6 @@ namespace {
 constexpr int KXB = kMlpXbStride;  // row stride (bf16) of the stored inputs
 constexpr int HS = H + 4;          // row stride (float) of pre-activations and dZ in shared memory
 constexpr int KX4 = (kMlpIn + 3) / 4 * 4;  // inputs rounded up to whole groups of four: 84
-
-// Wait for the preceding launch of the stream to complete (programmatic dependent launch: the
-// prologue before this runs beside its tail); no effect in an ordinary launch.
-__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // four BF16 at p (8-byte aligned) as floats
 __device__ __forceinline__ float4 bf4(const uint16_t *p)
@@ -651,22 +647,6 @@ AdamArgs adam_args(const MlpAdam &m)
     return o;
 }
 
-template <class... P, class... A>
-cudaError_t launch(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, bool dependent, A... args)
-{
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = dependent ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
-}
-
 template <int NR>
 constexpr size_t smem_outer() { return kMlpTile * ((KXB + H) * sizeof(uint16_t) + (3 * NR + 1) * sizeof(float)); }
 
@@ -674,8 +654,8 @@ cudaError_t launch_outer(const MlpWork &w, int slots, bool first, cudaStream_t s
 {
     // 8 units per CTA (8 CTAs per tile) while 16 would leave most SMs idle (a batch of 2048 rows: 128
     // CTAs against 64); 16 beyond: twice the multiply-adds per shared load
-    if (slots * 8 <= 2 * 152) return launch(k_mlp_outer<8>, dim3(8, slots), 224, smem_outer<8>(), s, true, w, first);
-    return launch(k_mlp_outer<16>, dim3(4, slots), 256, smem_outer<16>(), s, true, w, first);
+    if (slots * 8 <= 2 * 152) return launch_after(k_mlp_outer<8>, dim3(8, slots), 224, smem_outer<8>(), s, true, w, first);
+    return launch_after(k_mlp_outer<16>, dim3(4, slots), 256, smem_outer<16>(), s, true, w, first);
 }
 
 constexpr int kReduceBlocks = (kMlpParams + 127) / 128 + 1;
@@ -696,10 +676,10 @@ cudaError_t sample_pass(const MlpDev &net, const float *x, const float *t, const
         // 16 rows per CTA spread a minibatch over the SMs; 32 share one copy of the weights
         cudaError_t e;
         if (a.rows <= 152 * 2 * 16)
-            e = launch(k_mlp_rows<16>, dim3((unsigned)(a.rows / 16)), 128, sizeof(RowSmem<16, false>), s,
+            e = launch_after(k_mlp_rows<16>, dim3((unsigned)(a.rows / 16)), 128, sizeof(RowSmem<16, false>), s,
                        dependent || r0 > 0, net, a, w);
         else
-            e = launch(k_mlp_rows<32>, dim3((unsigned)std::min<int64_t>(a.rows / 32, 152 * 4)), 256,
+            e = launch_after(k_mlp_rows<32>, dim3((unsigned)std::min<int64_t>(a.rows / 32, 152 * 4)), 256,
                        sizeof(RowSmem<32, false>), s, dependent || r0 > 0, net, a, w);
         if (e != cudaSuccess) return e;
         if ((e = launch_outer(w, (int)(a.rows / kMlpTile), r0 == 0, s)) != cudaSuccess) return e;
@@ -738,7 +718,7 @@ cudaError_t mlp_loss_grad(const MlpDev &net, const float *x, const float *t, int
     int nb = 0;
     cudaError_t e = sample_pass(net, x, t, nullptr, n, w, nb, s, false);
     if (e != cudaSuccess) return e;
-    return launch(k_mlp_reduce<false>, dim3(kReduceBlocks), 128, 0, s, true, w.part, w.lsum, nb, (double)n, grad, loss,
+    return launch_after(k_mlp_reduce<false>, dim3(kReduceBlocks), 128, 0, s, true, w.part, w.lsum, nb, (double)n, grad, loss,
                   AdamArgs{});
 }
 
@@ -749,7 +729,7 @@ cudaError_t mlp_train_step(const MlpDev &net, const float *x, const float *t, co
     int nb = 0;
     cudaError_t e = sample_pass(net, x, t, idx, n, w, nb, s, dependent);
     if (e != cudaSuccess) return e;
-    return launch(k_mlp_reduce<true>, dim3(kReduceBlocks), 128, 0, s, true, w.part, w.lsum, nb, (double)n, nullptr,
+    return launch_after(k_mlp_reduce<true>, dim3(kReduceBlocks), 128, 0, s, true, w.part, w.lsum, nb, (double)n, nullptr,
                   loss, adam_args(adam));
 }
 
@@ -771,7 +751,7 @@ cudaError_t mlp_boundary_grad(const MlpDev &net, const BpttFields &f, const floa
         if (e == cudaSuccess) e = launch_outer(ww, (int)(rows / kMlpTile), r0 == 0, s);
     }
     if (e != cudaSuccess) return e;
-    return launch(k_mlp_reduce<false>, dim3(kReduceBlocks), 128, 0, s, true, w.part, (const double *)nullptr, nb, 1.0,
+    return launch_after(k_mlp_reduce<false>, dim3(kReduceBlocks), 128, 0, s, true, w.part, (const double *)nullptr, nb, 1.0,
                   grad, (double *)nullptr, AdamArgs{});
 }
 

@@ -39,8 +39,10 @@ struct ElementArgs {
     const float *rtab;
     // > 0: connectivity entries come from the caller and are checked against [0, n_check):
     // an entry outside is never read or written through (its gather reads 0, its scatter is
-    // dropped).  0: the library built the map, no checks.
+    // dropped).  0: the library built the map, no checks.  The coefficient table is then formed
+    // in the kernel, g_d * w_a * w_b in float (tab is not read).
     int64_t n_check;
+    float g[3], w[6];
 };
 
 struct UpdateArgs {

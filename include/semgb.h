@@ -314,8 +314,8 @@ int sem_batch_autotune(sem_batch *b, int *shots_per_cluster, int *warps_per_cta,
 /* ------------------------------------------------------------------------------------------
  * Groups of independent problems of uneven size (different meshes, orders, models, dt).  The
  * reference runs one problem per process (SEMproxy.cpp:41-64); a group advances several
- * solvers together, replaying one CUDA graph per two steps.  Two launch forms:
- *   SEM_GROUP_ONE_LAUNCH (default): each step is one source launch and one stencil-pass launch
+ * solvers together, replaying CUDA graphs of several steps.  Two launch forms:
+ *   SEM_GROUP_ONE_LAUNCH (default): each step is one stencil-pass launch (sources included)
  *     whose CTAs cover every member's tiles, so small members fill the SMs that large ones
  *     leave idle within the launch.  Needs every member on the stencil pass with order <= 4,
  *     the direct form and the default rounding; otherwise the group uses the branches.

@@ -54,9 +54,9 @@ struct sem_abc {
     float *d_hist_alt = nullptr;
     int hcur = 0;
     FaceDesc faces[6];
-    // two corrected steps replayed as one CUDA graph, per (current level, history buffer)
+    // kGraphSteps corrected steps replayed as one CUDA graph, per (current level, history buffer)
     // parity; valid while the solver's captured parameters are (graph_gen)
-    cudaGraphExec_t graph2[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
+    cudaGraphExec_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
     uint64_t graph_gen = 0;
     float *hist_now() const { return face && hcur ? d_hist_alt : d_hist; }
     float *hist_next() const { return face && !hcur ? d_hist_alt : d_hist; }
@@ -153,6 +153,40 @@ cudaError_t enqueue_correction(sem_abc *a)
     const Box &b = s->mesh->box;
     return abc_history(a->d_shell, a->n_shell, s->d_p[1 - s->cur], x.sx, x.sy, x.sz, b.nxp, b.nz, a->d_hist,
                        s->stream);
+}
+
+// No source node is read or written by the corrections: those reach the strip nodes' neighbours.
+// The passes of a run of steps can then add the next step's sources before the correction runs.
+bool sources_clear_of_strip(const sem_abc *a)
+{
+    const Box &b = a->s->mesh->box;
+    const int64_t reach = (int64_t)a->layer * b.order + 1;
+    for (int64_t q : a->s->src_group) {
+        const int64_t iy = q / (b.nxp * b.nz), r = q - iy * b.nxp * b.nz, iz = r / b.nxp, ix = r - iz * b.nxp;
+        if (std::min({ix, b.nx - 1 - ix, iy, b.ny - 1 - iy, iz, b.nz - 1 - iz}) <= reach) return false;
+    }
+    return true;
+}
+
+// n corrected steps from the current level and history buffer
+cudaError_t enqueue_corrected(sem_abc *a, int n)
+{
+    sem_solver *s = a->s;
+    const bool run = sources_clear_of_strip(a);
+    for (int k = 0; k < n; k++) {
+        StepExtra x;
+        if (run) {
+            x.advance = k == 0 ? n : 0;
+            x.step_off = k;
+            x.inject = k + 1 < n;
+        }
+        x.after = k > 0;
+        cudaError_t e = solver_enqueue_step(s, s->cur, nullptr, &x);
+        s->cur ^= 1;
+        if (e == cudaSuccess) e = enqueue_correction(a);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 }  // namespace
@@ -360,7 +394,7 @@ int sem_abc_destroy(sem_abc *a)
     // the solver may already be gone (handles closed in any order): wait for the device instead
     // of the solver's stream
     cudaDeviceSynchronize();
-    for (auto &row : a->graph2)
+    for (auto &row : a->graph)
         for (auto &g : row)
             if (g) cudaGraphExecDestroy(g);
     dfree(a->d_nodes);
@@ -495,25 +529,20 @@ int sem_abc_step(sem_abc *a, int n_steps)
     int rc = solver_prepare(s, n_steps);
     if (rc) return rc;
     if (a->graph_gen != s->graph_gen) {
-        for (auto &row : a->graph2)
+        for (auto &row : a->graph)
             for (auto &g : row)
                 if (g) { cudaGraphExecDestroy(g); g = nullptr; }
         a->graph_gen = s->graph_gen;
     }
     int done = 0;
-    while (n_steps - done >= 2) {
-        cudaGraphExec_t &ge = a->graph2[s->cur][a->hcur];
+    for (; n_steps - done >= kGraphSteps; done += kGraphSteps) {
+        cudaGraphExec_t &ge = a->graph[s->cur][a->hcur];
         if (!ge) {
-            // capture two corrected steps; the level and history parities come back to where
-            // they started
+            // an even number of steps: the level and history parities come back to where they
+            // started
             cudaGraph_t g = nullptr;
             CUDA_TRY(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-            cudaError_t e = cudaSuccess;
-            for (int k = 0; k < 2 && e == cudaSuccess; k++) {
-                e = solver_enqueue_step(s, s->cur);
-                s->cur ^= 1;
-                if (e == cudaSuccess) e = enqueue_correction(a);
-            }
+            const cudaError_t e = enqueue_corrected(a, kGraphSteps);
             const cudaError_t e2 = cudaStreamEndCapture(s->stream, &g);
             if (e != cudaSuccess || e2 != cudaSuccess) {
                 if (g) cudaGraphDestroy(g);
@@ -524,13 +553,8 @@ int sem_abc_step(sem_abc *a, int n_steps)
             if (e3 != cudaSuccess) return sem_fail(SEM_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e3));
         }
         CUDA_TRY(cudaGraphLaunch(ge, s->stream));
-        done += 2;
     }
-    for (; done < n_steps; done++) {
-        CUDA_TRY(solver_enqueue_step(s, s->cur));
-        s->cur ^= 1;
-        CUDA_TRY(enqueue_correction(a));
-    }
+    CUDA_TRY(enqueue_corrected(a, n_steps - done));
     s->steps_done += n_steps;
     return SEM_OK;
     GUARD_END

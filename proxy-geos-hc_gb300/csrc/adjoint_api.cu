@@ -91,21 +91,23 @@ cudaError_t enqueue_segment(sem_adjoint *a, int len)
     k_restore_segment<<<152 * 8, 256, 0, f->stream>>>(a->d_ckpt, a->d_seg, a->n_int, a->every, f->d_p[f->cur],
                                                         f->d_p[1 - f->cur], f->d_ctr);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    for (int n = 0; n < len; n++) {
+    auto record = [&](int n) {
         StepExtra x;
         x.mode = STENCIL_RECORD_KP;
         x.kp = a->d_kp + (size_t)n * lv;
-        if ((e = solver_enqueue_step(f, f->cur, nullptr, &x)) != cudaSuccess) return e;
-        f->cur ^= 1;
-    }
-    for (int n = len - 1; n >= 0; n--) {
+        return x;
+    };
+    if ((e = solver_enqueue_run(f, f->cur, len, record)) != cudaSuccess) return e;
+    f->cur ^= len & 1;
+    auto gradient = [&](int n) {
         StepExtra x;
         x.mode = STENCIL_GRADIENT;
-        x.kp = a->d_kp + (size_t)n * lv;
+        x.kp = a->d_kp + (size_t)(len - 1 - n) * lv;
         x.grad = a->d_grad;
-        if ((e = solver_enqueue_step(g, g->cur, nullptr, &x)) != cudaSuccess) return e;
-        g->cur ^= 1;
-    }
+        return x;
+    };
+    if ((e = solver_enqueue_run(g, g->cur, len, gradient)) != cudaSuccess) return e;
+    g->cur ^= len & 1;
     k_dec_int<<<1, 1, 0, f->stream>>>(a->d_seg);
     return cudaGetLastError();
 }

@@ -31,7 +31,7 @@ static int fail(int code, const std::string &msg) { return sem_fail(code, msg); 
 void solver_invalidate_graphs(sem_solver *s)
 {
     s->graph_gen++;
-    for (auto &g : s->graph2)
+    for (auto &g : s->graph)
         if (g) { cudaGraphExecDestroy(g); g = nullptr; }
 }
 
@@ -162,16 +162,31 @@ int solver_set_raw_sources(sem_solver *s, int n_src, const int64_t *nodes, const
     cudaStreamSynchronize(s->stream);
     solver_invalidate_graphs(s);
     dfree(s->d_src_node);
+    dfree(s->d_src_off);
+    dfree(s->d_src_perm);
     dfree(s->d_src_coef);
     dfree(s->d_wavelet);
     s->nsrc = n_src;
     s->nsamples = n_samples;
     s->src_node.assign(nodes, nodes + n_src);
     s->src_coef.assign(coef, coef + n_src);
-    std::vector<int64_t> sorted(nodes, nodes + n_src);
-    std::sort(sorted.begin(), sorted.end());
-    s->src_distinct = std::adjacent_find(sorted.begin(), sorted.end()) == sorted.end();
+    // sources on one node form a group, in source order
+    std::vector<int> perm(n_src), off;
+    std::iota(perm.begin(), perm.end(), 0);
+    std::stable_sort(perm.begin(), perm.end(), [&](int a, int b) { return nodes[a] < nodes[b]; });
+    s->src_group.clear();
+    for (int k = 0; k < n_src; k++)
+        if (k == 0 || nodes[perm[k]] != nodes[perm[k - 1]]) {
+            off.push_back(k);
+            s->src_group.push_back(nodes[perm[k]]);
+        }
+    off.push_back(n_src);
+    s->src_version++;
     if (n_src > 0) {
+        CUDA_TRY(dalloc(&s->d_src_off, off.size()));
+        CUDA_TRY(dalloc(&s->d_src_perm, n_src));
+        CUDA_TRY(cudaMemcpy(s->d_src_off, off.data(), off.size() * 4, cudaMemcpyHostToDevice));
+        CUDA_TRY(cudaMemcpy(s->d_src_perm, perm.data(), n_src * 4, cudaMemcpyHostToDevice));
         CUDA_TRY(dalloc(&s->d_src_node, n_src));
         CUDA_TRY(dalloc(&s->d_src_coef, n_src));
         CUDA_TRY(cudaMemcpy(s->d_src_node, nodes, n_src * 8, cudaMemcpyHostToDevice));
@@ -483,6 +498,8 @@ int sem_solver_destroy(sem_solver *s)
     dfree(s->d_sy);
     dfree(s->d_sz);
     dfree(s->d_src_node);
+    dfree(s->d_src_off);
+    dfree(s->d_src_perm);
     dfree(s->d_src_coef);
     dfree(s->d_wavelet);
     dfree(s->d_rec_node);
@@ -818,6 +835,10 @@ int solver_prepare(sem_solver *s, int64_t n_new)
             CUDA_TRY(stencil_set_receivers(*s->stencil, s->rec_sorted.data(), s->nrec, s->rec_version));
             solver_invalidate_graphs(s);
         }
+        if (s->stencil->src_version != s->src_version) {
+            CUDA_TRY(stencil_set_sources(*s->stencil, s->src_group, s->src_version));
+            solver_invalidate_graphs(s);
+        }
     }
     if (s->nrec > 0 && s->steps_done + n_new > s->trace_cap) {
         int64_t cap = std::max<int64_t>(s->steps_done + n_new, std::max<int64_t>(64, 2 * s->trace_cap));
@@ -836,6 +857,12 @@ int solver_prepare(sem_solver *s, int64_t n_new)
     return SEM_OK;
 }
 
+SourceTable solver_sources(const sem_solver *s)
+{
+    return SourceTable{s->d_src_node, s->d_src_coef, s->d_wavelet, s->d_src_off, s->d_src_perm,
+                       s->nsamples > 0 ? (int)s->src_group.size() : 0, s->nsamples};
+}
+
 // One step with the current level index c; the new level lands in 1-c.  Optional events time
 // the source, stiffness and update launches; `extra` selects an adjoint-support mode of the
 // stencil pass (its side buffers for this step).
@@ -844,13 +871,16 @@ cudaError_t solver_enqueue_step(sem_solver *s, int c, cudaEvent_t *ev, const Ste
     sem_mesh *m = s->mesh;
     const Box &b = m->box;
     cudaError_t e;
-    SourceArgs sa{s->d_p[c], s->d_src_node, s->d_src_coef, s->d_wavelet, s->nsamples > 0 ? s->nsrc : 0,
-                  s->nsamples, s->d_ctr, s->src_distinct ? 1 : 0};
+    const StepExtra plain;
+    const StepExtra &x = extra ? *extra : plain;
+    const SourceTable src = solver_sources(s);
     if (ev) cudaEventRecord(ev[0], s->stream);
-    if ((e = launch_source(sa, s->stream)) != cudaSuccess) return e;
+    if (x.advance > 0)
+        if ((e = launch_source(SourceArgs{s->d_p[c], src, s->d_ctr, x.advance}, s->stream, x.after)) != cudaSuccess)
+            return e;
     if (ev) cudaEventRecord(ev[1], s->stream);
     if (resolved_kernel(s) == SEM_KERNEL_ELEMENT) {
-        if (extra && extra->mode != STENCIL_PLAIN) return cudaErrorInvalidValue;  // stencil pass only
+        if (x.mode != STENCIL_PLAIN || x.advance != 1 || x.inject) return cudaErrorInvalidValue;  // stencil pass only
         ElementArgs ea{};
         ea.conn = m->d_conn;
         ea.p = s->d_p[c];
@@ -892,17 +922,37 @@ cudaError_t solver_enqueue_step(sem_solver *s, int c, cudaEvent_t *ev, const Ste
         ta.nrec = s->nrec;
         ta.traces = s->d_traces;
         ta.ctr = s->d_ctr;
-        int mode = STENCIL_PLAIN;
-        if (extra) {
-            mode = extra->mode;
-            ta.kp = extra->kp;
-            ta.grad = extra->grad;
-        }
+        ta.kp = x.kp;
+        ta.grad = x.grad;
+        ta.step_off = x.step_off;
+        ta.inject = x.inject ? 1 : 0;
+        ta.src = src;
+        ta.src_cta = s->stencil->d_src_cta;
+        // follows the source launch, or the pass before in a run of steps
+        const bool after = !ev && (x.advance > 0 || x.after);
         const bool direct = s->form == SEM_FORM_DIRECT || s->rounding == SEM_ROUNDING_REFERENCE;
-        if ((e = launch_stencil(*s->stencil, ta, c, s->sponge, s->stream, mode, direct)) != cudaSuccess) return e;
+        if ((e = launch_stencil(*s->stencil, ta, c, s->sponge, s->stream, x.mode, direct, after)) != cudaSuccess)
+            return e;
         if (ev) cudaEventRecord(ev[2], s->stream);
     }
     if (ev) cudaEventRecord(ev[3], s->stream);
+    return cudaSuccess;
+}
+
+cudaError_t solver_enqueue_run(sem_solver *s, int c, int n, const std::function<StepExtra(int)> &side)
+{
+    const bool element = resolved_kernel(s) == SEM_KERNEL_ELEMENT;  // its update adds no sources
+    for (int k = 0; k < n; k++, c ^= 1) {
+        StepExtra x = side ? side(k) : StepExtra{};
+        if (!element) {
+            x.advance = k == 0 ? n : 0;
+            x.step_off = k;
+            x.inject = k + 1 < n;
+            x.after = k > 0;
+        }
+        cudaError_t e = solver_enqueue_step(s, c, nullptr, &x);
+        if (e != cudaSuccess) return e;
+    }
     return cudaSuccess;
 }
 
@@ -912,15 +962,14 @@ static int build_graph(sem_solver *s, int c)
 {
     cudaGraph_t g = nullptr;
     CUDA_TRY(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-    cudaError_t e1 = solver_enqueue_step(s, c);
-    cudaError_t e2 = e1 == cudaSuccess ? solver_enqueue_step(s, 1 - c) : e1;
+    cudaError_t e2 = solver_enqueue_run(s, c, kGraphSteps);
     cudaError_t e3 = cudaStreamEndCapture(s->stream, &g);
     if (e2 != cudaSuccess || e3 != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
         return fail(SEM_ERR_CUDA, std::string("graph capture: ") +
                                       cudaGetErrorString(e2 != cudaSuccess ? e2 : e3));
     }
-    cudaError_t e4 = cudaGraphInstantiate(&s->graph2[c], g, 0);
+    cudaError_t e4 = cudaGraphInstantiate(&s->graph[c], g, 0);
     cudaGraphDestroy(g);
     if (e4 != cudaSuccess) return fail(SEM_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e4));
     return SEM_OK;
@@ -935,18 +984,16 @@ int sem_solver_step(sem_solver *s, int n_steps)
     int rc = solver_prepare(s, n_steps);
     if (rc) return rc;
     int done = 0;
-    while (n_steps - done >= 2) {
-        if (!s->graph2[s->cur]) {
+    for (; n_steps - done >= kGraphSteps; done += kGraphSteps) {  // an even number of swaps
+        if (!s->graph[s->cur]) {
             rc = build_graph(s, s->cur);
             if (rc) return rc;
         }
-        CUDA_TRY(cudaGraphLaunch(s->graph2[s->cur], s->stream));
-        done += 2;  // two swaps: the current level index is unchanged
+        CUDA_TRY(cudaGraphLaunch(s->graph[s->cur], s->stream));
     }
     if (done < n_steps) {
-        CUDA_TRY(solver_enqueue_step(s, s->cur));
-        s->cur ^= 1;
-        done++;
+        CUDA_TRY(solver_enqueue_run(s, s->cur, n_steps - done));
+        s->cur ^= (n_steps - done) & 1;
     }
     s->steps_done += n_steps;
     return SEM_OK;

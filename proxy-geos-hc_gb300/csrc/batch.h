@@ -24,11 +24,11 @@ struct BatchSourceArgs {
     const float *wavelet;  // [nshot][nsamples]
     int nshot, nsamples;
     int64_t shot_stride;
-    const int *ctr;
+    int *ctr;              // ctr[1] <- ctr[0] (this step), ctr[0] += advance
+    int advance;           // steps until the next source launch
 };
 
-// Adds every shot's source sample of the current step, then advances the step counter
-// (ctr[1] = step of the level being written, ctr[0] = next step).
-cudaError_t launch_batch_source(const BatchSourceArgs &a, int *ctr, cudaStream_t st);
+// Adds every shot's source sample of the current step and advances the step counter.
+cudaError_t launch_batch_source(const BatchSourceArgs &a, cudaStream_t st);
 
 }  // namespace semgb

@@ -13,7 +13,7 @@
 
 #include "abi.h"
 #include "batch.h"
-#include "stencil.h"
+#include "solver.h"
 
 using namespace semgb;
 
@@ -48,14 +48,14 @@ struct sem_batch {
     StencilTables *st = nullptr;
     BatchTuning tune;
     bool tuned = false;
-    cudaGraphExec_t graph2[2] = {nullptr, nullptr};
+    cudaGraphExec_t graph[2] = {nullptr, nullptr};  // [parity] kGraphSteps steps
 };
 
 namespace {
 
 void invalidate(sem_batch *b)
 {
-    for (auto &g : b->graph2)
+    for (auto &g : b->graph)
         if (g) { cudaGraphExecDestroy(g); g = nullptr; }
 }
 
@@ -76,13 +76,21 @@ StencilArgs args_for(const sem_batch *b, int c, bool record)
     return a;
 }
 
-cudaError_t enqueue(sem_batch *b, int c)
+// n steps from level c: one source launch, then the passes, each adding the sources of the step
+// after it.
+cudaError_t enqueue(sem_batch *b, int c, int n)
 {
-    BatchSourceArgs sa{b->d_p[c], b->d_src_node, b->d_src_coef, b->d_wavelet, b->nsamples > 0 ? b->nshot : 0,
-                       b->nsamples, b->n_int, b->d_ctr};
-    cudaError_t e = launch_batch_source(sa, b->d_ctr, b->stream);
-    if (e != cudaSuccess) return e;
-    return launch_stencil(*b->st, args_for(b, c, true), c, b->sponge, b->stream);
+    const int nsrc = b->nsamples > 0 ? b->nshot : 0;
+    cudaError_t e = launch_batch_source(BatchSourceArgs{b->d_p[c], b->d_src_node, b->d_src_coef, b->d_wavelet, nsrc,
+                                                        b->nsamples, b->n_int, b->d_ctr, n}, b->stream);
+    for (int k = 0; k < n && e == cudaSuccess; k++, c ^= 1) {
+        StencilArgs a = args_for(b, c, true);
+        a.step_off = k;
+        a.inject = k + 1 < n;
+        a.src = SourceTable{b->d_src_node, b->d_src_coef, b->d_wavelet, nullptr, nullptr, nsrc, b->nsamples};
+        e = launch_stencil(*b->st, a, c, b->sponge, b->stream, STENCIL_PLAIN, true, true);
+    }
+    return e;
 }
 
 // Sets the stencil pass's y-chunk (planes per CTA) and regroups the receivers by CTA.
@@ -345,27 +353,25 @@ int sem_batch_step(sem_batch *b, int n_steps)
     int rc = prepare(b, n_steps);
     if (rc) return rc;
     int done = 0;
-    while (n_steps - done >= 2) {
-        if (!b->graph2[b->cur]) {
+    for (; n_steps - done >= kGraphSteps; done += kGraphSteps) {
+        if (!b->graph[b->cur]) {
             cudaGraph_t g = nullptr;
             CUDA_TRY(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-            cudaError_t e1 = enqueue(b, b->cur);
-            cudaError_t e2 = e1 == cudaSuccess ? enqueue(b, 1 - b->cur) : e1;
+            cudaError_t e2 = enqueue(b, b->cur, kGraphSteps);
             cudaError_t e3 = cudaStreamEndCapture(b->stream, &g);
             if (e2 != cudaSuccess || e3 != cudaSuccess) {
                 if (g) cudaGraphDestroy(g);
                 return sem_fail(SEM_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e2 != cudaSuccess ? e2 : e3));
             }
-            cudaError_t e4 = cudaGraphInstantiate(&b->graph2[b->cur], g, 0);
+            cudaError_t e4 = cudaGraphInstantiate(&b->graph[b->cur], g, 0);
             cudaGraphDestroy(g);
             if (e4 != cudaSuccess) return sem_fail(SEM_ERR_CUDA, cudaGetErrorString(e4));
         }
-        CUDA_TRY(cudaGraphLaunch(b->graph2[b->cur], b->stream));
-        done += 2;
+        CUDA_TRY(cudaGraphLaunch(b->graph[b->cur], b->stream));
     }
     if (done < n_steps) {
-        CUDA_TRY(enqueue(b, b->cur));
-        b->cur ^= 1;
+        CUDA_TRY(enqueue(b, b->cur, n_steps - done));
+        b->cur ^= (n_steps - done) & 1;
     }
     b->steps_done += n_steps;
     return SEM_OK;

@@ -1,10 +1,10 @@
 // group_api.cu -- many independent problems of uneven size advanced together (sem_group_*).
 //
 // Each member is an ordinary solver (its own mesh, order, model, dt, sources and receivers).
-// Two ways to advance them, both replayed from one CUDA graph per two steps:
+// Two ways to advance them, both replayed from CUDA graphs of kGraphSteps steps (fewer: enqueued):
 //  - one launch (default where every member allows it: stencil pass, orders 1-4, direct form,
-//    default rounding): per step one source launch and one pass launch over all members' CTAs
-//    (k_group.cu).  The members' tiles are cut along y into chunks of about the same number of
+//    default rounding): one pass launch per step over all members' CTAs (k_group.cu), sources
+//    launched once per run of steps and added by the passes between.  The members' tiles are cut along y into chunks of about the same number of
 //    planes, chosen for the whole group, and the longest CTAs come first in the launch;
 //  - branches: the group stream forks into the members' streams, each branch holds that member's
 //    own steps (source, stencil pass), and the branches join back; largest member first.
@@ -31,7 +31,7 @@ struct sem_group {
     std::vector<cudaEvent_t> join;
     int want = SEM_GROUP_ONE_LAUNCH;   // requested launch form
     int form = -1;                     // form of the graphs and state below
-    cudaGraphExec_t graph[2] = {nullptr, nullptr};  // [f]: two steps starting at parity f
+    cudaGraphExec_t graph[2] = {nullptr, nullptr};  // [f]: kGraphSteps steps starting at parity f
     std::vector<uint64_t> gen;         // members' graph generations at build
     std::vector<int> cur0;             // member's current level at parity 0
     int flip = 0;                      // parity of the next step
@@ -91,23 +91,21 @@ cudaError_t enqueue_branches(sem_group *g, int steps, int parity)
     for (size_t i = 0; i < g->members.size(); i++) {
         sem_solver *s = g->members[i];
         if ((e = cudaStreamWaitEvent(s->stream, g->fork, 0)) != cudaSuccess) return e;
-        int c = g->cur0[i] ^ parity;
-        for (int k = 0; k < steps; k++, c ^= 1)
-            if ((e = solver_enqueue_step(s, c)) != cudaSuccess) return e;
+        if ((e = solver_enqueue_run(s, g->cur0[i] ^ parity, steps)) != cudaSuccess) return e;
         if ((e = cudaEventRecord(g->join[i], s->stream)) != cudaSuccess) return e;
         if ((e = cudaStreamWaitEvent(g->stream, g->join[i], 0)) != cudaSuccess) return e;
     }
     return cudaSuccess;
 }
 
+// One source launch, then the passes, each adding the sources of the step after it.
 cudaError_t enqueue_one_launch(sem_group *g, int steps, int parity)
 {
-    for (int k = 0; k < steps; k++) {
-        cudaError_t e = semgb::launch_group_step(g->d_mem, (int)g->members.size(), g->d_cta_member, g->n_ctas,
-                                                 g->max_order, parity ^ (k & 1), g->stream);
-        if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
+    cudaError_t e = semgb::launch_group_source(g->d_mem, (int)g->members.size(), parity, steps, g->stream);
+    for (int k = 0; k < steps && e == cudaSuccess; k++)
+        e = semgb::launch_group_pass(g->d_mem, g->d_cta_member, g->n_ctas, g->max_order, parity ^ (k & 1), k,
+                                     k + 1 < steps, g->stream);
+    return e;
 }
 
 cudaError_t enqueue(sem_group *g, int steps, int parity)
@@ -119,7 +117,7 @@ int capture(sem_group *g, int parity)
 {
     cudaGraph_t graph = nullptr;
     CUDA_TRY(cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal));
-    cudaError_t e1 = enqueue(g, 2, parity);
+    cudaError_t e1 = enqueue(g, kGraphSteps, parity);
     cudaError_t e2 = cudaStreamEndCapture(g->stream, &graph);
     if (e1 != cudaSuccess || e2 != cudaSuccess) {
         if (graph) cudaGraphDestroy(graph);
@@ -220,8 +218,9 @@ int write_descriptors(sem_group *g)
             a.nrec = s->nrec;
             a.traces = s->d_traces;
             a.ctr = s->d_ctr;
-            m.src[k] = semgb::SourceArgs{s->d_p[c], s->d_src_node, s->d_src_coef, s->d_wavelet,
-                                         s->nsamples > 0 ? s->nsrc : 0, s->nsamples, s->d_ctr, s->src_distinct ? 1 : 0};
+            a.src = solver_sources(s);
+            a.src_cta = t.d_src_cta;
+            m.src[k] = semgb::SourceArgs{s->d_p[c], a.src, s->d_ctr, 0};
         }
         const int64_t nc = (int64_t)t.grid[0] * t.grid[1] * t.grid[2];
         if (cta + nc > (int64_t)0x7fffffff) return sem_fail(SEM_ERR_ARG, "group too large for one launch");
@@ -269,6 +268,7 @@ int build_one_launch(sem_group *g)
         t->ychunk = chunks[i];
         t->grid[2] = (int)((t->ny + chunks[i] - 1) / chunks[i]);
         CUDA_TRY(semgb::stencil_set_receivers(*t, s->rec_sorted.data(), s->nrec, s->rec_version));
+        CUDA_TRY(semgb::stencil_set_sources(*t, s->src_group, s->src_version));
         if (!s->sponge && !g->ones[i]) {
             const Box &b = s->mesh->box;
             const size_t len = (size_t)std::max(b.nx, std::max(b.ny, b.nz));
@@ -385,18 +385,19 @@ int sem_group_step(sem_group *g, int n_steps)
         CUDA_TRY(cudaStreamWaitEvent(g->stream, g->join[i], 0));
     }
     int done = 0;
-    while (n_steps - done >= 2) {
+    for (; n_steps - done >= kGraphSteps; done += kGraphSteps) {
         if (!g->graph[g->flip]) {
             int rc = capture(g, g->flip);
             if (rc) return rc;
         }
         CUDA_TRY(cudaGraphLaunch(g->graph[g->flip], g->stream));
-        done += 2;
     }
     if (done < n_steps) {
-        CUDA_TRY(enqueue(g, 1, g->flip));
-        for (sem_solver *s : g->members) s->cur ^= 1;
-        g->flip ^= 1;
+        CUDA_TRY(enqueue(g, n_steps - done, g->flip));
+        if ((n_steps - done) & 1) {
+            for (sem_solver *s : g->members) s->cur ^= 1;
+            g->flip ^= 1;
+        }
     }
     // and the members' later calls (reads, solo steps) after this work
     CUDA_TRY(cudaEventRecord(g->fork, g->stream));

@@ -4,7 +4,7 @@
 // Every member keeps its own levels, tensor maps and tiling; the launch's CTAs are the members'
 // tiles x y-chunks one after another (cta_member maps a CTA to its member), so the GPU's
 // scheduler fills SMs with whatever CTAs are left of any member, and a step of the whole group
-// is two launches (sources, then the pass) instead of two per member.  A CTA runs the same code
+// is one launch (the pass, which also adds the next step's sources) instead of one per member.  A CTA runs the same code
 // as the single-box pass of its order (stencil_body.cuh), so each member's results are bit for
 // bit those of the member stepped alone.  The CTA has kGroupThreads threads; at order 3 (three
 // warps) the fourth warp only takes part in the barriers.
@@ -39,31 +39,23 @@ __device__ __forceinline__ void tensormap_acquire(const CUtensorMap *m)
                  : "memory");
 }
 
-// Sources of every member (block m: member m), as k_source does for one box: sources on distinct
-// nodes added by all threads, otherwise by one thread in source order; the member's step
-// counter advanced.
-__global__ void k_group_source(const GroupMember *__restrict__ mem, int k)
+// Sources of every member (block m: member m), as k_source does for one box.
+__global__ void k_group_source(const GroupMember *__restrict__ mem, int k, int advance)
 {
     const SourceArgs &a = mem[blockIdx.x].src[k];
+    grid_launch_dependents();
     const int n = a.ctr[0];
     __syncthreads();  // every thread has read the step before thread 0 advances the counter
-    if (n < a.nsamples) {
-        if (a.distinct) {
-            for (int i = threadIdx.x; i < a.nsrc; i += blockDim.x)
-                a.cur[a.node[i]] += a.coef[i] * a.wavelet[(int64_t)i * a.nsamples + n];
-        } else if (threadIdx.x == 0) {
-            for (int i = 0; i < a.nsrc; i++)
-                a.cur[a.node[i]] += a.coef[i] * a.wavelet[(int64_t)i * a.nsamples + n];
-        }
-    }
+    if (n < a.t.nsamples)
+        for (int u = threadIdx.x; u < a.t.ngroup; u += blockDim.x) add_source_group(a.t, u, n, a.cur);
     if (threadIdx.x == 0) {
         a.ctr[1] = n;
-        a.ctr[0] = n + 1;
+        a.ctr[0] = n + advance;
     }
 }
 
 __global__ void __launch_bounds__(kGroupThreads, kGroupMinBlocks)
-    k_group(const GroupMember *__restrict__ mem, const int *__restrict__ cta_member, int k)
+    k_group(const GroupMember *__restrict__ mem, const int *__restrict__ cta_member, int k, int step_off, int inject)
 {
     const GroupMember &g = mem[__ldg(cta_member + blockIdx.x)];
     const StencilTables &t = g.t;
@@ -81,15 +73,15 @@ __global__ void __launch_bounds__(kGroupThreads, kGroupMinBlocks)
     const StencilArgs &a = g.a[k];
     const NoClassTable none{};
     switch (g.order) {
-    case 1: stencil_cta<1, true, STENCIL_PLAIN, true, false, false, true>(rmap, wmap, pmap, amap, t, a, none, 0, bx, bz, chunk); break;
-    case 2: stencil_cta<2, true, STENCIL_PLAIN, true, false, false, true>(rmap, wmap, pmap, amap, t, a, none, 0, bx, bz, chunk); break;
-    case 3: stencil_cta<3, true, STENCIL_PLAIN, true, false, false, true>(rmap, wmap, pmap, amap, t, a, none, 0, bx, bz, chunk); break;
+    case 1: stencil_cta<1, true, STENCIL_PLAIN, true, false, false, true>(rmap, wmap, pmap, amap, t, a, none, 0, bx, bz, chunk, step_off, inject != 0); break;
+    case 2: stencil_cta<2, true, STENCIL_PLAIN, true, false, false, true>(rmap, wmap, pmap, amap, t, a, none, 0, bx, bz, chunk, step_off, inject != 0); break;
+    case 3: stencil_cta<3, true, STENCIL_PLAIN, true, false, false, true>(rmap, wmap, pmap, amap, t, a, none, 0, bx, bz, chunk, step_off, inject != 0); break;
     default:
         if (t.shape == kTileSquare)
             stencil_cta<4, true, STENCIL_PLAIN, true, false, false, true, kSquareRW>(rmap, wmap, pmap, amap, t, a, none, 0,
-                                                                                     bx, bz, chunk);
+                                                                                     bx, bz, chunk, step_off, inject != 0);
         else
-            stencil_cta<4, true, STENCIL_PLAIN, true, false, false, true>(rmap, wmap, pmap, amap, t, a, none, 0, bx, bz, chunk);
+            stencil_cta<4, true, STENCIL_PLAIN, true, false, false, true>(rmap, wmap, pmap, amap, t, a, none, 0, bx, bz, chunk, step_off, inject != 0);
         break;
     }
 }
@@ -133,16 +125,19 @@ int group_blocks_per_sm(int max_order)
     return n;
 }
 
-cudaError_t launch_group_step(const GroupMember *members, int n_members, const int *cta_member, int n_ctas,
-                              int max_order, int k, cudaStream_t s)
+cudaError_t launch_group_source(const GroupMember *members, int n_members, int k, int advance, cudaStream_t s)
 {
-    if (n_members < 1 || n_ctas < 1 || max_order < 1 || max_order > kGroupMaxOrder || (k & ~1))
-        return cudaErrorInvalidValue;
-    k_group_source<<<n_members, 256, 0, s>>>(members, k);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    k_group<<<n_ctas, kGroupThreads, smem_upto(max_order), s>>>(members, cta_member, k);
+    if (n_members < 1 || (k & ~1)) return cudaErrorInvalidValue;
+    k_group_source<<<n_members, 256, 0, s>>>(members, k, advance);
     return cudaGetLastError();
+}
+
+cudaError_t launch_group_pass(const GroupMember *members, const int *cta_member, int n_ctas, int max_order, int k,
+                              int step_off, bool inject, cudaStream_t s)
+{
+    if (n_ctas < 1 || max_order < 1 || max_order > kGroupMaxOrder || (k & ~1)) return cudaErrorInvalidValue;
+    return launch_after(k_group, dim3((unsigned)n_ctas), kGroupThreads, smem_upto(max_order), s, true, members,
+                        cta_member, k, step_off, inject ? 1 : 0);
 }
 
 }  // namespace semgb

@@ -12,6 +12,7 @@
 #include <vector>
 #include <cstddef>
 
+#include "launch.cuh"
 #include "mlp_device.cuh"
 
 namespace semgb {
@@ -314,6 +315,7 @@ __global__ void __launch_bounds__(128, 3) k_abc_face(const MlpDev net, const Abc
     load_net(s, net);
     // the depth plane outside the box stays zero for every tile
     for (int i = threadIdx.x; i < 3 * kPD; i += blockDim.x) patch[(i / kPD) * kPL + i % kPD] = 0.f;
+    grid_dependency_wait();  // launched as a dependent of the step: the weights staged beside its tail
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
     const int64_t plane = a.nxp * a.nz;
     // A tile stages the face and inside planes of the three levels with a one-node rim: a thread
@@ -587,8 +589,7 @@ cudaError_t abc_face(const MlpDev &net, const AbcFaceArgs &a, cudaStream_t s)
     cudaError_t e = resident_ctas(k_abc_face, sm, cache, resident);
     if (e != cudaSuccess) return e;
     // persistent CTAs, as many as are resident at once (the weights are staged once per CTA)
-    k_abc_face<<<(unsigned)std::min<int64_t>(a.ntiles, resident), T, sm, s>>>(net, a);
-    return cudaGetLastError();
+    return launch_after(k_abc_face, dim3((unsigned)std::min<int64_t>(a.ntiles, resident)), T, sm, s, true, net, a);
 }
 
 cudaError_t abc_apply(const AbcArgs &a, float *p_new, float *hist, cudaStream_t s)

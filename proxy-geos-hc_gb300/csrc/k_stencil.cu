@@ -36,7 +36,7 @@ template <int O, bool SPONGE, int MODE, bool DIRECT, bool MULTI, bool REF = fals
 __global__ void __launch_bounds__(Cfg<O, RWS>::THREADS, Cfg<O, RWS>::MIN_BLOCKS)
     k_stencil(const __grid_constant__ CUtensorMap ring_map, const __grid_constant__ CUtensorMap win_map,
               const __grid_constant__ CUtensorMap prev_map, const __grid_constant__ CUtensorMap a_map,
-              const StencilTables t, const StencilArgs a, const __grid_constant__ ClassParam<O, REF> ct)
+              const StencilBox t, const StencilArgs a, const __grid_constant__ ClassParam<O, REF> ct)
 {
     // CTA -> (x-tile, z-tile, y-chunk): grid (x-tiles, z-tiles, chunks).  MULTI (many shots, the
     // levels stacking the shots along y: plane p of shot s is plane s*ny + p): grid
@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(Cfg<O, RWS>::THREADS, Cfg<O, RWS>::MIN_BLOCKS)
         chunk = (int)blockIdx.z;
     }
     stencil_cta<O, SPONGE, MODE, DIRECT, MULTI, REF, false, RWS>(&ring_map, &win_map, &prev_map, &a_map, t, a, ct,
-                                                                 shot, bx, bz, chunk);
+                                                                 shot, bx, bz, chunk, a.step_off, a.inject != 0);
 }
 
 template <int O, int RWS = SEM_STENCIL_RW>
@@ -104,7 +104,7 @@ int blocks_per_sm(int order, int shape)
 
 template <int O, bool SPONGE, int MODE, bool DIRECT, bool MULTI, bool REF = false, int RWS = SEM_STENCIL_RW>
 void launch_om(const dim3 &grid, const LevelMaps &cm, const LevelMaps &pm, const StencilTables &t,
-               const StencilArgs &a, cudaStream_t s)
+               const StencilArgs &a, cudaStream_t s, bool after)
 {
     using C = Cfg<O, RWS>;
     ClassParam<O, REF> ct{};
@@ -129,12 +129,13 @@ void launch_om(const dim3 &grid, const LevelMaps &cm, const LevelMaps &pm, const
                            a, ct);
         return;
     }
-    k_stencil<O, SPONGE, MODE, DIRECT, MULTI, REF, RWS>
-        <<<grid, C::THREADS, C::SMEM, s>>>(cm.tile, cm.win, pm.tile, t.amap, t, a, ct);
+    launch_after(k_stencil<O, SPONGE, MODE, DIRECT, MULTI, REF, RWS>, grid, C::THREADS, C::SMEM, s, after, cm.tile,
+                 cm.win, pm.tile, t.amap, t, a, ct);
 }
 
 template <int O, bool DIRECT>
-cudaError_t launch_of(const StencilTables &t, const StencilArgs &a, int ci, bool sponge, int mode, cudaStream_t s)
+cudaError_t launch_of(const StencilTables &t, const StencilArgs &a, int ci, bool sponge, int mode, cudaStream_t s,
+                      bool after)
 {
     const LevelMaps &cm = t.lv[ci], &pm = t.lv[1 - ci];
     if (t.shape == kTileSquare) {
@@ -142,8 +143,8 @@ cudaError_t launch_of(const StencilTables &t, const StencilArgs &a, int ci, bool
         if constexpr (O == 4) {
             if (t.class_tab || t.nshot != 1 || mode != STENCIL_PLAIN) return cudaErrorInvalidValue;
             const dim3 grid(t.grid[0], t.grid[1], t.grid[2]);
-            if (sponge) launch_om<O, true, STENCIL_PLAIN, DIRECT, false, false, kSquareRW>(grid, cm, pm, t, a, s);
-            else launch_om<O, false, STENCIL_PLAIN, DIRECT, false, false, kSquareRW>(grid, cm, pm, t, a, s);
+            if (sponge) launch_om<O, true, STENCIL_PLAIN, DIRECT, false, false, kSquareRW>(grid, cm, pm, t, a, s, after);
+            else launch_om<O, false, STENCIL_PLAIN, DIRECT, false, false, kSquareRW>(grid, cm, pm, t, a, s, after);
             return cudaGetLastError();
         }
         return cudaErrorInvalidValue;
@@ -154,12 +155,12 @@ cudaError_t launch_of(const StencilTables &t, const StencilArgs &a, int ci, bool
             if (mode != STENCIL_PLAIN) return cudaErrorInvalidValue;
             if (t.nshot > 1) {
                 const dim3 grid((unsigned)((int64_t)t.grid[0] * t.grid[1] * t.nshot), (unsigned)t.grid[2]);
-                if (sponge) launch_om<O, true, STENCIL_PLAIN, true, true, true>(grid, cm, pm, t, a, s);
-                else launch_om<O, false, STENCIL_PLAIN, true, true, true>(grid, cm, pm, t, a, s);
+                if (sponge) launch_om<O, true, STENCIL_PLAIN, true, true, true>(grid, cm, pm, t, a, s, after);
+                else launch_om<O, false, STENCIL_PLAIN, true, true, true>(grid, cm, pm, t, a, s, after);
             } else {
                 const dim3 grid(t.grid[0], t.grid[1], t.grid[2]);
-                if (sponge) launch_om<O, true, STENCIL_PLAIN, true, false, true>(grid, cm, pm, t, a, s);
-                else launch_om<O, false, STENCIL_PLAIN, true, false, true>(grid, cm, pm, t, a, s);
+                if (sponge) launch_om<O, true, STENCIL_PLAIN, true, false, true>(grid, cm, pm, t, a, s, after);
+                else launch_om<O, false, STENCIL_PLAIN, true, false, true>(grid, cm, pm, t, a, s, after);
             }
             return cudaGetLastError();
         }
@@ -170,20 +171,20 @@ cudaError_t launch_of(const StencilTables &t, const StencilArgs &a, int ci, bool
         if constexpr (DIRECT) {
             if (mode != STENCIL_PLAIN) return cudaErrorInvalidValue;
             const dim3 grid((unsigned)((int64_t)t.grid[0] * t.grid[1] * t.nshot), (unsigned)t.grid[2]);
-            if (sponge) launch_om<O, true, STENCIL_PLAIN, true, true>(grid, cm, pm, t, a, s);
-            else launch_om<O, false, STENCIL_PLAIN, true, true>(grid, cm, pm, t, a, s);
+            if (sponge) launch_om<O, true, STENCIL_PLAIN, true, true>(grid, cm, pm, t, a, s, after);
+            else launch_om<O, false, STENCIL_PLAIN, true, true>(grid, cm, pm, t, a, s, after);
             return cudaGetLastError();
         }
         return cudaErrorInvalidValue;
     }
     const dim3 grid(t.grid[0], t.grid[1], t.grid[2]);
     switch (mode * 2 + (sponge ? 1 : 0)) {
-    case 0: launch_om<O, false, STENCIL_PLAIN, DIRECT, false>(grid, cm, pm, t, a, s); break;
-    case 1: launch_om<O, true, STENCIL_PLAIN, DIRECT, false>(grid, cm, pm, t, a, s); break;
-    case 2: launch_om<O, false, STENCIL_RECORD_KP, DIRECT, false>(grid, cm, pm, t, a, s); break;
-    case 3: launch_om<O, true, STENCIL_RECORD_KP, DIRECT, false>(grid, cm, pm, t, a, s); break;
-    case 4: launch_om<O, false, STENCIL_GRADIENT, DIRECT, false>(grid, cm, pm, t, a, s); break;
-    case 5: launch_om<O, true, STENCIL_GRADIENT, DIRECT, false>(grid, cm, pm, t, a, s); break;
+    case 0: launch_om<O, false, STENCIL_PLAIN, DIRECT, false>(grid, cm, pm, t, a, s, after); break;
+    case 1: launch_om<O, true, STENCIL_PLAIN, DIRECT, false>(grid, cm, pm, t, a, s, after); break;
+    case 2: launch_om<O, false, STENCIL_RECORD_KP, DIRECT, false>(grid, cm, pm, t, a, s, after); break;
+    case 3: launch_om<O, true, STENCIL_RECORD_KP, DIRECT, false>(grid, cm, pm, t, a, s, after); break;
+    case 4: launch_om<O, false, STENCIL_GRADIENT, DIRECT, false>(grid, cm, pm, t, a, s, after); break;
+    case 5: launch_om<O, true, STENCIL_GRADIENT, DIRECT, false>(grid, cm, pm, t, a, s, after); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
@@ -191,9 +192,10 @@ cudaError_t launch_of(const StencilTables &t, const StencilArgs &a, int ci, bool
 
 template <int O>
 cudaError_t launch_o(const StencilTables &t, const StencilArgs &a, int ci, bool sponge, int mode, bool direct,
-                     cudaStream_t s)
+                     cudaStream_t s, bool after)
 {
-    return direct ? launch_of<O, true>(t, a, ci, sponge, mode, s) : launch_of<O, false>(t, a, ci, sponge, mode, s);
+    return direct ? launch_of<O, true>(t, a, ci, sponge, mode, s, after)
+                  : launch_of<O, false>(t, a, ci, sponge, mode, s, after);
 }
 
 template <int O, bool SPONGE, int MODE, bool DIRECT, bool MULTI = false, bool REF = false, int RWS = SEM_STENCIL_RW>
@@ -336,6 +338,14 @@ int stencil_bind(StencilTables &t, const float *p0, const float *p1, const float
     return 0;
 }
 
+// CTA (tile and y-chunk) that owns a device-layout node
+static int64_t owner_cta(const StencilTables &t, int64_t n)
+{
+    const int64_t nxz = t.nxp * t.nz;
+    const int64_t y = n / nxz, rem = n - y * nxz, z = rem / t.nxp, x = rem - z * t.nxp;
+    return x / t.tile_x + t.grid[0] * (z / t.tile_z + t.grid[1] * (y / t.ychunk));
+}
+
 cudaError_t stencil_set_receivers(StencilTables &t, const int64_t *sorted_nodes, int nrec, uint64_t version)
 {
     if (t.d_rec_off) { cudaFree(t.d_rec_off); t.d_rec_off = nullptr; }
@@ -345,11 +355,8 @@ cudaError_t stencil_set_receivers(StencilTables &t, const int64_t *sorted_nodes,
     const int64_t ncta = (int64_t)t.grid[0] * t.grid[1] * t.grid[2];
     std::vector<int64_t> owner(nrec);
     std::vector<int> count(ncta + 1, 0);
-    const int64_t nxz = t.nxp * t.nz;
     for (int r = 0; r < nrec; r++) {
-        const int64_t n = sorted_nodes[r];
-        const int64_t y = n / nxz, rem = n - y * nxz, z = rem / t.nxp, x = rem - z * t.nxp;
-        owner[r] = x / t.tile_x + t.grid[0] * (z / t.tile_z + t.grid[1] * (y / t.ychunk));
+        owner[r] = owner_cta(t, sorted_nodes[r]);
         count[owner[r] + 1]++;
     }
     for (int64_t c = 0; c < ncta; c++) count[c + 1] += count[c];
@@ -361,6 +368,18 @@ cudaError_t stencil_set_receivers(StencilTables &t, const int64_t *sorted_nodes,
     if ((e = cudaMemcpy(t.d_rec_off, count.data(), (ncta + 1) * sizeof(int), cudaMemcpyHostToDevice)) != cudaSuccess)
         return e;
     return cudaMemcpy(t.d_rec_idx, idx.data(), nrec * sizeof(int), cudaMemcpyHostToDevice);
+}
+
+cudaError_t stencil_set_sources(StencilTables &t, const std::vector<int64_t> &group_nodes, uint64_t version)
+{
+    if (t.d_src_cta) { cudaFree(t.d_src_cta); t.d_src_cta = nullptr; }
+    t.src_version = version;
+    if (group_nodes.empty()) return cudaSuccess;
+    std::vector<int> cta(group_nodes.size());
+    for (size_t u = 0; u < cta.size(); u++) cta[u] = (int)owner_cta(t, group_nodes[u]);
+    cudaError_t e = cudaMalloc(&t.d_src_cta, cta.size() * sizeof(int));
+    if (e != cudaSuccess) return e;
+    return cudaMemcpy(t.d_src_cta, cta.data(), cta.size() * sizeof(int), cudaMemcpyHostToDevice);
 }
 
 int stencil_set_class_table(StencilTables &t, const float *tab)
@@ -380,6 +399,7 @@ void stencil_tables_free(StencilTables *&t)
     delete[] t->class_tab;
     if (t->d_rec_off) cudaFree(t->d_rec_off);
     if (t->d_rec_idx) cudaFree(t->d_rec_idx);
+    if (t->d_src_cta) cudaFree(t->d_src_cta);
     delete t;
     t = nullptr;
 }
@@ -403,15 +423,15 @@ cudaError_t stencil_kernel_setup()
 }
 
 cudaError_t launch_stencil(const StencilTables &t, const StencilArgs &a, int cur_index, bool sponge, cudaStream_t s,
-                           int mode, bool direct)
+                           int mode, bool direct, bool after)
 {
     if (mode != STENCIL_PLAIN && (!a.kp || (mode == STENCIL_GRADIENT && !a.grad))) return cudaErrorInvalidValue;
     switch (t.order) {
-    case 1: return launch_o<1>(t, a, cur_index, sponge, mode, direct, s);
-    case 2: return launch_o<2>(t, a, cur_index, sponge, mode, direct, s);
-    case 3: return launch_o<3>(t, a, cur_index, sponge, mode, direct, s);
-    case 4: return launch_o<4>(t, a, cur_index, sponge, mode, direct, s);
-    case 5: return launch_o<5>(t, a, cur_index, sponge, mode, direct, s);
+    case 1: return launch_o<1>(t, a, cur_index, sponge, mode, direct, s, after);
+    case 2: return launch_o<2>(t, a, cur_index, sponge, mode, direct, s, after);
+    case 3: return launch_o<3>(t, a, cur_index, sponge, mode, direct, s, after);
+    case 4: return launch_o<4>(t, a, cur_index, sponge, mode, direct, s, after);
+    case 5: return launch_o<5>(t, a, cur_index, sponge, mode, direct, s, after);
     default: return cudaErrorInvalidValue;
     }
 }

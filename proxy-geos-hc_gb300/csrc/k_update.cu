@@ -11,30 +11,25 @@
 #include <algorithm>
 
 #include "kernels.h"
+#include "launch.cuh"
 
 namespace semgb {
 
 namespace {
 
-// One block.  Sources on distinct nodes are added by all threads (one addition per node, the
-// same bits as any order); otherwise one thread adds them in source order, as the reference's
-// loop does, so that sources sharing a node sum in that order.
+// One block: the sources of step ctr[0], one thread per node (in source order on a node, as the
+// reference's loop sums them).
 __global__ void k_source(const SourceArgs a)
 {
+    grid_launch_dependents();
+    grid_dependency_wait();
     const int n = a.ctr[0];
     __syncthreads();  // every thread has read the step before thread 0 advances the counter
-    if (n < a.nsamples) {
-        if (a.distinct) {
-            for (int k = threadIdx.x; k < a.nsrc; k += blockDim.x)
-                a.cur[a.node[k]] += a.coef[k] * a.wavelet[(int64_t)k * a.nsamples + n];
-        } else if (threadIdx.x == 0) {
-            for (int k = 0; k < a.nsrc; k++)
-                a.cur[a.node[k]] += a.coef[k] * a.wavelet[(int64_t)k * a.nsamples + n];
-        }
-    }
+    if (n < a.t.nsamples)
+        for (int u = threadIdx.x; u < a.t.ngroup; u += blockDim.x) add_source_group(a.t, u, n, a.cur);
     if (threadIdx.x == 0) {
         a.ctr[1] = n;
-        a.ctr[0] = n + 1;
+        a.ctr[0] = n + a.advance;
     }
 }
 
@@ -259,10 +254,9 @@ cudaError_t launch_mass_ref(float *m, const float *vel, int ex, int ey, int ez, 
     return cudaGetLastError();
 }
 
-cudaError_t launch_source(const SourceArgs &a, cudaStream_t s)
+cudaError_t launch_source(const SourceArgs &a, cudaStream_t s, bool after)
 {
-    k_source<<<1, a.distinct && a.nsrc > 32 ? 256 : 32, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_after(k_source, dim3(1), a.t.ngroup > 32 ? 256 : 32, 0, s, after, a);
 }
 
 cudaError_t launch_connectivity(int32_t *conn, int ex, int ey, int ez, int order, int64_t nxp,

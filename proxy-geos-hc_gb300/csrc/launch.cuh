@@ -9,7 +9,10 @@ namespace semgb {
 // Wait for the preceding launch of the stream to complete, its writes visible; no effect in an
 // ordinary launch.  Nothing that earlier work wrote may be read before.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// Let the next launch of the stream start once every CTA of this one has started.
+// Let the next launch of the stream start once every CTA of this one has started (without it: once
+// they have exited).  Only for launches that leave SMs idle: the passes of the step, which fill
+// them, measured slower with it (the waiting CTAs of the next pass take the slots and issue time of
+// the running ones: 6.4 against 4.7 us per step on 40^3 elements of order 2).
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Launch; dependent: as a programmatic dependent of the preceding kernel of the stream.

@@ -4,10 +4,18 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <functional>
 #include <vector>
 
 #include "abi.h"
 #include "stencil.h"
+
+// Steps per captured graph (even: the level parity returns).  Inside one, passes follow each other
+// as programmatic dependents and only the first step has a source launch; between graphs the
+// launch gap is that of an ordinary kernel boundary.  Per step, against two steps (four kernels) per
+// graph: 40^3 elements of order 2 7.3 -> 4.7 us, 61 x 70 x 53 of order 4 52.5 -> 49.0, 80 x 77 x 83
+// of order 5 304.7 -> 291.9, 200^3 of order 4 1394.6 -> 1392.2, a group of 32 small boxes 36.7 -> 34.1.
+constexpr int kGraphSteps = 16;
 
 struct sem_solver {
     sem_mesh *mesh = nullptr;
@@ -35,8 +43,10 @@ struct sem_solver {
     float *d_sx = nullptr, *d_sy = nullptr, *d_sz = nullptr;
     // sources
     int nsrc = 0, nsamples = 0;
-    bool src_distinct = true;  // no two sources on one node
     int64_t *d_src_node = nullptr;
+    int *d_src_off = nullptr, *d_src_perm = nullptr;  // sources grouped by node (SourceTable)
+    std::vector<int64_t> src_group;                   // node of each group
+    uint64_t src_version = 1;
     float *d_src_coef = nullptr;
     float *d_wavelet = nullptr;
     std::vector<int64_t> src_node;
@@ -55,8 +65,8 @@ struct sem_solver {
     int *d_upd_rec_off = nullptr;   // receivers grouped by update-kernel block
     uint64_t upd_rec_version = 0;
     int64_t steps_done = 0;
-    // graphs: [parity] two steps starting at level `parity`
-    cudaGraphExec_t graph2[2] = {nullptr, nullptr};
+    // graphs: [parity] kGraphSteps steps starting at level `parity`
+    cudaGraphExec_t graph[2] = {nullptr, nullptr};
     uint64_t graph_gen = 0;  // bumped whenever captured launch parameters may have changed
 };
 
@@ -65,6 +75,11 @@ struct StepExtra {
     int mode = semgb::STENCIL_PLAIN;
     float *kp = nullptr;
     float *grad = nullptr;
+    // place in a run of steps: steps the source launch covers (0: the pass before added this
+    // step's sources), steps since it, whether this pass adds the next step's, and whether the
+    // preceding kernel on the stream belongs to the run
+    int advance = 1, step_off = 0;
+    bool inject = false, after = false;
 };
 
 // Device resources for stepping n_new more steps (mass, stencil tables, receiver CSR, trace
@@ -72,8 +87,11 @@ struct StepExtra {
 int solver_prepare(sem_solver *s, int64_t n_new);
 // One step from level c (source, stiffness + update, receivers) enqueued on the solver stream.
 cudaError_t solver_enqueue_step(sem_solver *s, int c, cudaEvent_t *ev = nullptr, const StepExtra *extra = nullptr);
+// n steps from level c with nothing between them.  side(k) (may be empty) gives step k's side buffers.
+cudaError_t solver_enqueue_run(sem_solver *s, int c, int n, const std::function<StepExtra(int)> &side = nullptr);
 void solver_invalidate_graphs(sem_solver *s);
 // Sources by device-layout node with explicit coefficients: p^n[node_k] += coef_k * wavelet_k[n].
+semgb::SourceTable solver_sources(const sem_solver *s);
 int solver_set_raw_sources(sem_solver *s, int n_src, const int64_t *nodes, const float *coef, const float *wavelet,
                            int n_samples);
 // A field between the device layout (rows of nxp floats) and a host array in the reference

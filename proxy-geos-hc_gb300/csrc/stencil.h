@@ -14,6 +14,8 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <vector>
+
 #include "host_util.h"
 #include "kernels.h"
 
@@ -36,23 +38,29 @@ struct alignas(16) ClassTable {
 // that single-shot plain steps may take (the 64 x 16 default wastes more lanes on some boxes)
 enum StencilTileShape { kTileDefault = 0, kTileSquare = 1 };
 
-struct StencilTables {
+// What a CTA of the pass needs of a box: the kernel's parameter (the whole tables as a parameter,
+// tensor maps included, made every parameter access of the plane loop about 1 % dearer at 801^3
+// nodes once they grew past 1.6 KB: 1393 -> 1408 us per launch).
+struct StencilBox {
+    int64_t nx = 0, nxp = 0, ny = 0, nz = 0;
+    int64_t shot_stride = 0;  // floats per shot field: nxp * nz * ny
+    float g[3] = {0, 0, 0};   // g_d = |detJ| / J_dd^2 for x (xi1), z (xi2), y (xi3)
+    int grid[3] = {0, 0, 0};  // tiles along x, z and y-chunks (launch: x * z * nshot CTAs by chunks)
+    int nshot = 1;            // shots stacked along y in the levels (many-shot form)
+    int ychunk = 0;           // planes per CTA
+};
+
+struct StencilTables : StencilBox {
     int order = 0;
     int shape = kTileDefault;  // tile shape the kernels and the tables below are built for
     // SEM_ROUNDING_REFERENCE: the reference's assembled node-class coefficients, host memory
     // owned by the tables (null: the tensor-product operator below)
     float *class_tab = nullptr;
-    int64_t nx = 0, nxp = 0, ny = 0, nz = 0;
-    float g[3] = {0, 0, 0};   // g_d = |detJ| / J_dd^2 for x (xi1), z (xi2), y (xi3)
     float wa[6] = {0};        // assembled weight by local index: wa[0] = 2 w_0, wa[l] = w_l
     int tile_x = 0, tile_z = 0, halo_x = 0;
     int threads = 0;          // per CTA
-    int grid[3] = {0, 0, 0};  // tiles along x, z and y-chunks (launch: x * z * nshot CTAs by chunks)
-    int nshot = 1;            // shots stacked along y in the levels (many-shot form)
     int cluster = 1;          // many-shot form: CTAs of consecutive shots of a tile co-scheduled as
                               // one thread-block cluster (divides nshot; 1: plain launch)
-    int64_t shot_stride = 0;  // floats per shot field: nxp * nz * ny
-    int ychunk = 0;           // planes per CTA
     size_t smem = 0;          // dynamic shared memory per CTA
     LevelMaps lv[2];          // per pressure buffer
     CUtensorMap amap;         // dt^2/M, tile boxes
@@ -62,6 +70,8 @@ struct StencilTables {
     int *d_rec_off = nullptr;
     int *d_rec_idx = nullptr;
     uint64_t rec_version = 0;
+    int *d_src_cta = nullptr;   // CTA that owns each source group's node
+    uint64_t src_version = 0;
 };
 
 struct StencilArgs {
@@ -74,7 +84,15 @@ struct StencilArgs {
     const int *rec_idx;
     int nrec;
     float *traces;
-    const int *ctr;
+    const int *ctr;            // the pass's step is ctr[1] + step_off
+    int step_off;
+    // inject: after its stores (and receiver samples) a CTA adds the next step's sources on its own
+    // nodes to the new level, so a run of steps needs one source launch at its start.
+    // src_cta[u]: the CTA that owns group u's node (many shots: src.node[shot] is the shot's node,
+    // -1: none, and src.off, src.perm and src_cta are not read)
+    int inject;
+    SourceTable src;
+    const int *src_cta;
     int *status;               // set non-zero when a bounded wait gives up
     // adjoint support (device layout, one value per node; unused by the plain step):
     //   STENCIL_RECORD_KP: kp <- (K p^n) on interior nodes, 0 elsewhere
@@ -91,7 +109,7 @@ constexpr int kGroupMaxOrder = 4;
 struct GroupMember {  // 128-byte aligned, as its tensor maps
     StencilTables t;    // tensor maps of the member's levels, its tiling with the group's y-chunks
     StencilArgs a[2];   // [k]: pass arguments at group parity k (current level cur0 ^ k)
-    SourceArgs src[2];  // [k]: source arguments at group parity k
+    SourceArgs src[2];  // [k]: source arguments at group parity k (advance: set by the launch)
     int order;
     int cur0;           // index of the member's current level at parity 0
     int cta0;           // the member's first CTA in the launch
@@ -104,10 +122,13 @@ cudaError_t group_kernel_setup();
 constexpr int kGroupThreads = 128;
 size_t group_smem(int max_order);
 int group_blocks_per_sm(int max_order);
-// One step of every member: sources, then the pass (receivers included).  cta_member[c] is the
-// member of CTA c; members[m].cta0 its first CTA.
-cudaError_t launch_group_step(const GroupMember *members, int n_members, const int *cta_member, int n_ctas,
-                              int max_order, int k, cudaStream_t s);
+// Sources of every member's next step; the counters advance by `advance` steps.
+cudaError_t launch_group_source(const GroupMember *members, int n_members, int k, int advance, cudaStream_t s);
+// The pass of every member (receivers included), step_off steps after the last source launch;
+// inject: with the next step's sources.  cta_member[c] is the member of CTA c; members[m].cta0
+// its first CTA.  Launched as a programmatic dependent of the preceding kernel of the stream.
+cudaError_t launch_group_pass(const GroupMember *members, const int *cta_member, int n_ctas, int max_order, int k,
+                              int step_off, bool inject, cudaStream_t s);
 
 // Tables and tiling for a box (no device buffers yet).  Returns 0 or a cudaError_t.
 // nshot > 1: the many-shot form, levels holding nshot fields one after another (traces
@@ -121,6 +142,8 @@ void stencil_tile_dims(int order, int shape, int &tx, int &tz, int &hx, int &thr
 int stencil_bind(StencilTables &t, const float *p0, const float *p1, const float *a);
 // Group node-sorted receivers (device-layout indices) by owning CTA (device CSR in t).
 cudaError_t stencil_set_receivers(StencilTables &t, const int64_t *sorted_nodes, int nrec, uint64_t version);
+// Owning CTA of each source group (group_nodes: its node, device layout), for StencilArgs::src_cta.
+cudaError_t stencil_set_sources(StencilTables &t, const std::vector<int64_t> &group_nodes, uint64_t version);
 // Switch the pass to the reference-rounding operator with node-class table `tab` (layout of
 // reference_class_table, copied), or back to the tensor-product operator (tab null).
 int stencil_set_class_table(StencilTables &t, const float *tab);
@@ -130,7 +153,8 @@ cudaError_t stencil_kernel_setup();
 // direct: operator form sum_d T_d p_{i+d} with the diagonal T_0 = -sum_{d!=0} T_d (fewer
 // instructions); otherwise the difference form sum_{d!=0} T_d (p_{i+d} - p_i), exactly zero on a
 // constant field.
+// after: as a programmatic dependent of the preceding kernel of the stream.
 cudaError_t launch_stencil(const StencilTables &t, const StencilArgs &a, int cur_index, bool sponge,
-                           cudaStream_t s, int mode = STENCIL_PLAIN, bool direct = true);
+                           cudaStream_t s, int mode = STENCIL_PLAIN, bool direct = true, bool after = false);
 
 }  // namespace semgb

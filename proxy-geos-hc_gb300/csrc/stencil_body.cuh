@@ -9,6 +9,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "launch.cuh"
 #include "stencil.h"
 #include "tma.cuh"
 
@@ -333,9 +334,9 @@ using ClassParam = typename std::conditional<REF, ClassTable<O>, NoClassTable>::
 // orders); the extra threads take part in the barriers only.
 template <int O, bool SPONGE, int MODE, bool DIRECT, bool MULTI, bool REF, bool GROUP, int RWS = SEM_STENCIL_RW>
 __device__ __forceinline__ void stencil_cta(const CUtensorMap *rmap, const CUtensorMap *wmap, const CUtensorMap *pmap,
-                                            const CUtensorMap *amap, const StencilTables &t, const StencilArgs &a,
+                                            const CUtensorMap *amap, const StencilBox &t, const StencilArgs &a,
                                             const ClassParam<O, REF> &ct, const int shot, const int bx, const int bz,
-                                            const int chunk)
+                                            const int chunk, const int step_off, const bool inject)
 {
     static_assert(!REF || DIRECT, "the reference-rounding operator is a direct form");
     using C = Cfg<O, RWS>;
@@ -375,6 +376,8 @@ __device__ __forceinline__ void stencil_cta(const CUtensorMap *rmap, const CUten
     }
     __syncthreads();
     if (threadIdx.x == 0) {
+        // the levels are read, and any of them written, only after the preceding launch has finished
+        grid_dependency_wait();
         for (int p = yb - O; p <= min(yb + O + kLook - 1, ye - 1 + O); p++) issue_ring(p);
         for (int p = yb; p <= min(yb + kLook - 1, ye - 1); p++) issue_aux(p);
     }
@@ -419,6 +422,7 @@ __device__ __forceinline__ void stencil_cta(const CUtensorMap *rmap, const CUten
     const int64_t plane_stride = nxp * t.nz;
     const int64_t group_stride = (int64_t)GR * nxp;
 
+    grid_dependency_wait();
     bool ok = true;
     for (int p = yb - O; p < yb + O; p++) {
         const int i = p - yb + O;  // < 2O < R: first fill of each of these slots
@@ -655,17 +659,35 @@ __device__ __forceinline__ void stencil_cta(const CUtensorMap *rmap, const CUten
             }
         return;
     }
+    const int cta = bx + t.grid[0] * (bz + t.grid[1] * chunk);  // tile and chunk
     if (a.nrec > 0) {
-        const int cta = bx + t.grid[0] * (bz + t.grid[1] * chunk);  // tile and chunk
         const int r0 = a.rec_off[cta], r1 = a.rec_off[cta + 1];
         if (r0 < r1) {  // uniform over the CTA; its new values are visible after the last barrier
-            const int step = a.ctr[1];
+            const int step = a.ctr[1] + step_off;
             const float *lvl = a.prev + (MULTI ? (int64_t)shot * t.shot_stride : 0);
             for (int r = r0 + (int)threadIdx.x; r < r1; r += GROUP ? (int)blockDim.x : C::THREADS) {
                 const int j = a.rec_idx[r];
                 // traces [step][receiver][shot]
                 const int64_t k = (int64_t)step * a.nrec + a.rec_perm[j];
                 a.traces[MULTI ? k * t.nshot + shot : k] = lvl[a.rec_node[j]];
+            }
+        }
+    }
+    if (inject && a.src.ngroup > 0) {
+        const int n = a.ctr[1] + step_off + 1;
+        __syncthreads();  // the receivers above have sampled the level without the next sources
+        if (n < a.src.nsamples) {
+            float *lvl = a.prev + (MULTI ? (int64_t)shot * t.shot_stride : 0);
+            if constexpr (MULTI) {
+                const int64_t q = a.src.node[shot];
+                if (threadIdx.x == 0 && q >= 0) {
+                    const int64_t plane = t.nxp * t.nz, y = q / plane, r = q - y * plane, zz = r / t.nxp, x = r - zz * t.nxp;
+                    if (x / TX == bx && zz / TZ == bz && y / t.ychunk == chunk)
+                        lvl[q] += a.src.coef[shot] * a.src.wavelet[(int64_t)shot * a.src.nsamples + n];
+                }
+            } else {
+                for (int u = (int)threadIdx.x; u < a.src.ngroup; u += GROUP ? (int)blockDim.x : C::THREADS)
+                    if (a.src_cta[u] == cta) add_source_group(a.src, u, n, lvl);
             }
         }
     }

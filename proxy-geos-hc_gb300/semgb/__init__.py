@@ -541,8 +541,8 @@ class Batch:
 
 
 class Group:
-    """Independent solvers of uneven size advanced together (sem_group_*), one CUDA graph per
-    two steps: by default one launch per step over every member's tiles (GROUP_ONE_LAUNCH),
+    """Independent solvers of uneven size advanced together (sem_group_*), replayed from
+    CUDA graphs: by default one launch per step over every member's tiles (GROUP_ONE_LAUNCH),
     or each member's own launches as parallel branches (GROUP_BRANCHES)."""
 
     def __init__(self, solvers, launch: int = 0):

@@ -591,44 +591,56 @@ int sem_abc_bptt(sem_abc *a, int n_steps, int n_roi, const int64_t *roi_nodes, c
     // work arrays (freed on every exit path)
     float *rec = nullptr, *dx = nullptr;
     float *A[3] = {nullptr, nullptr, nullptr}, *v = nullptr, *dref = nullptr;
-    int *sidx = nullptr;
+    int *sidx = nullptr, *ridx = nullptr;
     int64_t *droi = nullptr;
     double *dloss = nullptr;
+    const int64_t dx_stride = (nb + 31) / 32 * 32;
     auto release = [&]() {
         cudaStreamSynchronize(st);
         dfree(rec); dfree(dx);
         for (auto &p : A) dfree(p);
-        dfree(v); dfree(dref); dfree(sidx); dfree(droi); dfree(dloss);
+        dfree(v); dfree(dref); dfree(sidx); dfree(ridx); dfree(droi); dfree(dloss);
     };
     cudaError_t e = dalloc(&rec, (size_t)(n_steps + 2) * n_int);
-    if (e == cudaSuccess) e = dalloc(&dx, (size_t)nb * kMlpIn);
-    if (e == cudaSuccess && grad) e = ensure_work(a->net, nb);
-    for (auto &p : A)
-        if (e == cudaSuccess) e = dalloc(&p, (size_t)n_int);
-    if (e == cudaSuccess) e = dalloc(&v, (size_t)n_int);
     if (e == cudaSuccess && n_roi > 0) e = dalloc(&dref, (size_t)n_steps * n_roi);
-    if (e == cudaSuccess) e = dalloc(&sidx, (size_t)n_int);
     if (e == cudaSuccess && n_roi > 0) e = dalloc(&droi, (size_t)n_roi);
-    if (e == cudaSuccess) e = dalloc(&dloss, 1);
-    if (e == cudaSuccess) {
+    if (e == cudaSuccess) e = dalloc(&dloss, (size_t)n_steps);
+    if (grad) {
+        if (e == cudaSuccess) e = dalloc(&dx, (size_t)dx_stride * kMlpIn);
+        if (e == cudaSuccess) e = ensure_work(a->net, mlp_boundary_groups(nb) * mlp_work_rows(nb));
+        for (auto &p : A)
+            if (e == cudaSuccess) e = dalloc(&p, (size_t)n_int);
+        if (e == cudaSuccess) e = dalloc(&v, (size_t)n_int);
+        if (e == cudaSuccess) e = dalloc(&sidx, (size_t)n_int);
         std::vector<int64_t> nodes(nb);
-        e = cudaMemcpy(nodes.data(), a->d_nodes, nb * 8, cudaMemcpyDeviceToHost);
+        if (e == cudaSuccess) e = cudaMemcpy(nodes.data(), a->d_nodes, nb * 8, cudaMemcpyDeviceToHost);
         std::vector<int> map(n_int, -1);
         for (int64_t i = 0; i < nb; i++) map[nodes[i]] = (int)i;
         if (e == cudaSuccess) e = cudaMemcpy(sidx, map.data(), n_int * 4, cudaMemcpyHostToDevice);
+        std::fill(map.begin(), map.end(), -1);
+        bool twice = false;
+        for (int r = 0; r < n_roi; r++) {
+            twice = twice || map[roi[r]] >= 0;
+            map[roi[r]] = r;
+        }
+        if (!twice && n_roi > 0) {
+            if (e == cudaSuccess) e = dalloc(&ridx, (size_t)n_int);
+            if (e == cudaSuccess) e = cudaMemcpy(ridx, map.data(), n_int * 4, cudaMemcpyHostToDevice);
+        }
     }
     if (e == cudaSuccess && n_roi > 0) e = cudaMemcpy(droi, roi.data(), n_roi * 8, cudaMemcpyHostToDevice);
     if (e == cudaSuccess && n_roi > 0)
         e = cudaMemcpy(dref, ref, (size_t)n_steps * n_roi * 4, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemsetAsync(dloss, 0, 8, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(rec, 0, 2 * n_int * 4, st);  // p^{-1} = p^0 = 0: from rest
-    // forward, the levels after every step recorded
+    // forward, the levels after every step recorded (by a kernel: the chain of dependent launches
+    // goes on)
     for (int m = 1; m <= n_steps && e == cudaSuccess; m++) {
-        e = solver_enqueue_step(s, s->cur);
+        StepExtra x;
+        x.after = m > 1;
+        e = solver_enqueue_step(s, s->cur, nullptr, &x);
         s->cur ^= 1;
         if (e == cudaSuccess) e = enqueue_correction(a);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(rec + (size_t)(m + 1) * n_int, s->d_p[s->cur], n_int * 4, cudaMemcpyDeviceToDevice, st);
+        if (e == cudaSuccess) e = bptt_copy_level(s->d_p[s->cur], rec + (size_t)(m + 1) * n_int, n_int, st);
     }
     s->steps_done += n_steps;
     BpttFields f{};
@@ -638,16 +650,14 @@ int sem_abc_bptt(sem_abc *a, int n_steps, int n_roi, const int64_t *roi_nodes, c
     f.sy = s->sponge ? s->d_sy : nullptr;
     f.sz = s->sponge ? s->d_sz : nullptr;
     f.nodes = a->d_nodes; f.nb = nb; f.sidx = sidx;
-    f.dx = dx;
+    f.shell = a->d_shell; f.n_shell = a->n_shell;
+    f.dx = dx; f.dx_stride = dx_stride; f.ridx = ridx;
     for (int k = 0; k < 3; k++) f.a[k] = A[k];
     f.v = v; f.roi = droi; f.n_roi = n_roi;
-    for (auto p : A)
-        if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, n_int * 4, st);
-    if (!grad) {
-        // the loss only
-        for (int m = 1; m <= n_steps && e == cudaSuccess; m++)
-            e = bptt_loss(f, rec + (size_t)(m + 1) * n_int, dref + (size_t)(m - 1) * n_roi, dloss, st);
-    } else {
+    if (e == cudaSuccess && n_roi > 0) e = bptt_losses(f, rec + 2 * n_int, n_int, dref, n_steps, dloss, st);
+    if (grad) {
+        for (auto p : A)
+            if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, n_int * 4, st);
         BpttOperator op{};
         op.order = b.order;
         Gll gl;
@@ -665,24 +675,36 @@ int sem_abc_bptt(sem_abc *a, int n_steps, int n_roi, const int64_t *roi_nodes, c
         for (int k = 0; k < 3; k++) op.g[k] = s->stencil->g[k];
         sem_mlp *net = a->net;
         if (e == cudaSuccess) e = cudaMemsetAsync(net->d_grad, 0, kMlpParams * 4, st);
+        auto level = [&](int m) { return rec + (size_t)(m + 1) * n_int; };
+        auto ref_of = [&](int m) { return dref + (size_t)(m - 1) * n_roi; };
+        const int groups = mlp_boundary_groups(nb);
+        int group = 0;
+        if (e == cudaSuccess) e = bptt_seed(f, level(n_steps), ref_of(n_steps), st);
         for (int m = n_steps; m >= 1 && e == cudaSuccess; m--) {
-            const float *lm = rec + (size_t)(m + 1) * n_int, *lm1 = rec + (size_t)m * n_int,
-                        *lm2 = rec + (size_t)(m - 1) * n_int;
-            e = bptt_loss(f, lm, dref + (size_t)(m - 1) * n_roi, dloss, st);
-            if (e == cudaSuccess) e = mlp_boundary_grad(net->dev(), f, lm, lm1, lm2, net->d_grad, net->work, st);
-            if (e == cudaSuccess) e = bptt_scatter(f, st);
-            if (e == cudaSuccess) e = bptt_interior(f, op, s->d_a, st);
+            e = mlp_boundary_rows(net->dev(), f, level(m), level(m - 1), level(m - 2), group++, net->work, net->d_grad, st);
+            if (e == cudaSuccess && (group == groups || m == 1)) {
+                e = mlp_boundary_params(nb, group, net->d_grad, net->work, st);
+                group = 0;
+            }
+            if (e == cudaSuccess) e = bptt_scatter(f, s->d_a, st);
+            const bool fused = ridx && m > 1;
+            if (e == cudaSuccess)
+                e = bptt_interior(f, op, fused ? level(m - 1) : nullptr, fused ? ref_of(m - 1) : nullptr, st);
             // the adjoints move one level back: out^{m-1} becomes the newest
-            float *old = f.a[0];
-            f.a[0] = f.a[1];
-            f.a[1] = f.a[2];
-            f.a[2] = old;
-            if (e == cudaSuccess) e = cudaMemsetAsync(old, 0, n_int * 4, st);
+            std::swap(f.a[0], f.a[1]);
+            std::swap(f.a[1], f.a[2]);
+            if (e == cudaSuccess && !ridx && m > 1) e = bptt_seed(f, level(m - 1), ref_of(m - 1), st);
         }
         if (e == cudaSuccess) e = cudaMemcpyAsync(grad, net->d_grad, kMlpParams * 4, cudaMemcpyDeviceToHost, st);
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(loss, dloss, 8, cudaMemcpyDeviceToHost, st);
+    std::vector<double> step_loss(n_steps, 0.0);
+    if (e == cudaSuccess && n_roi > 0)
+        e = cudaMemcpyAsync(step_loss.data(), dloss, (size_t)n_steps * 8, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (grad) std::reverse(step_loss.begin(), step_loss.end());  // (summed newest step first, as the sweep runs)
+    double sum = 0.0;
+    for (double l : step_loss) sum += l;
+    if (e == cudaSuccess) *loss = sum;
     release();
     CUDA_TRY(e);
     return SEM_OK;

@@ -22,8 +22,9 @@
 // 7.6 + 6.5 + 7.6 us for the three launches under the profiler, which adds about 3 us to each.
 // Bound by latency: one warp per scheduler in dependent phases (stage, two MMA layers, GELU, dZ),
 // not by bytes (0.66 MB of samples) or multiply-adds (27 M).  The adjoint's pass over 13,826
-// boundary nodes: 26.7 + 14.7 + 11.5 us against 350 us for the separate feature, forward,
-// gradient and feature-gradient kernels; there the row kernel issues on half of all cycles.
+// boundary nodes: 25 us for the rows and, the entries and sums of five steps taken together, 10 + 3
+// us per step, against 350 us for the separate feature, forward, gradient and feature-gradient
+// kernels; there the row kernel issues on half of all cycles and waits on its phase barriers.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -39,6 +40,7 @@ namespace {
 constexpr int KXB = kMlpXbStride;  // row stride (bf16) of the stored inputs
 constexpr int HS = H + 4;          // row stride (float) of pre-activations and dZ in shared memory
 constexpr int KX4 = (kMlpIn + 3) / 4 * 4;  // inputs rounded up to whole groups of four: 84
+constexpr int DXS = KX4 + 1;               // row stride of the feature gradient in shared memory
 
 // four BF16 at p (8-byte aligned) as floats
 __device__ __forceinline__ float4 bf4(const uint16_t *p)
@@ -100,7 +102,7 @@ struct RowSmem {
     float d[NROW];
     // boundary: features (then inputs), feature gradient, per-row scale, arg-max, node coordinates
     alignas(16) float xf[BOUNDARY ? NROW * KX4 : 4];
-    alignas(16) float dx[BOUNDARY ? NROW * KX4 : 4];
+    alignas(16) float dx[BOUNDARY ? NROW * (KX4 + 1) : 4];
     float scale[BOUNDARY ? NROW : 1], gb[BOUNDARY ? NROW : 1], y[BOUNDARY ? NROW : 1];
     int kstar[BOUNDARY ? NROW : 1];
     int4 at[BOUNDARY ? NROW : 1];
@@ -289,8 +291,9 @@ __global__ void __launch_bounds__(8 * NROW, 3) k_mlp_boundary(const MlpDev net, 
     extern __shared__ __align__(16) unsigned char smem[];
     RowSmem<NROW, true> &s = *reinterpret_cast<RowSmem<NROW, true> *>(smem);
     const int tid = threadIdx.x;
-    copy_net(s.net, net);
+    copy_net(s.net, net);  // constant over the time loop: staged before the wait
     copies_landed();
+    grid_dependency_wait();
     const int64_t plane = f.nxp * f.nz;
     for (int64_t rg = (int64_t)blockIdx.x * NROW; rg < rows; rg += (int64_t)gridDim.x * NROW) {
         __syncthreads();  // the previous rows are stored
@@ -391,13 +394,14 @@ __global__ void __launch_bounds__(8 * NROW, 3) k_mlp_boundary(const MlpDev net, 
             }
 #pragma unroll
             for (int i = 0; i < 4; i++)
-                *reinterpret_cast<float4 *>(s.dx + (r + i) * KX4 + k) = make_float4(d[i][0], d[i][1], d[i][2], d[i][3]);
+#pragma unroll
+                for (int j = 0; j < 4; j++) s.dx[(r + i) * DXS + k + j] = d[i][j];
         }
         __syncthreads();
         // feature gradient in place of dx: the division by the scale, and the scale's own share
         if (tid < NROW && row0 + rg + tid < f.nb) {
             const float *xr = s.xf + tid * KX4;
-            float *d = s.dx + tid * KX4;
+            float *d = s.dx + tid * DXS;
             const int ks = s.kstar[tid];
             if (ks < 0) {
                 for (int k = 0; k < kMlpIn; k++) d[k] = 0.f;
@@ -415,9 +419,10 @@ __global__ void __launch_bounds__(8 * NROW, 3) k_mlp_boundary(const MlpDev net, 
             }
         }
         __syncthreads();
+        // (feature-major: the gather reads neighbouring boundary nodes together)
         for (int i = tid; i < NROW * kMlpIn; i += 8 * NROW) {
-            const int r = i / kMlpIn, k = i - r * kMlpIn;
-            if (row0 + rg + r < f.nb) f.dx[(row0 + rg + r) * kMlpIn + k] = s.dx[r * KX4 + k];
+            const int k = i / NROW, r = i - k * NROW;
+            if (row0 + rg + r < f.nb) f.dx[k * f.dx_stride + row0 + rg + r] = s.dx[r * DXS + k];
         }
     }
 }
@@ -462,26 +467,32 @@ __global__ void __launch_bounds__(NR == 16 ? 256 : 224) k_mlp_outer(const MlpWor
         const float *pd = (l1 ? s1 : s2) + un;
         const uint16_t *pk = (l1 ? sx : sh) + k;
         const int st = l1 ? KXB : H;
-        float a[UN][4];
+        // units in pairs, packed f32x2 (each half rounds as the scalar fused multiply-add)
+        float2 a[UN / 2][4];
 #pragma unroll
-        for (int i = 0; i < UN; i++)
+        for (int i = 0; i < UN / 2; i++)
 #pragma unroll
-            for (int j = 0; j < 4; j++) a[i][j] = 0.f;
-#pragma unroll 8
+            for (int j = 0; j < 4; j++) a[i][j] = make_float2(0.f, 0.f);
+#pragma unroll 4
         for (int r = 0; r < kMlpTile; r++) {
             const float4 v = bf4(pk);
-            float d[UN];
-            if constexpr (UN == 4) {
-                const float4 t = *reinterpret_cast<const float4 *>(pd);
-                d[0] = t.x; d[1] = t.y; d[2] = t.z; d[3] = t.w;
+            float2 d[UN / 2];
+            if constexpr (UN == 2) {
+                d[0] = *reinterpret_cast<const float2 *>(pd);
             } else {
-                const float2 t = *reinterpret_cast<const float2 *>(pd);
-                d[0] = t.x; d[1] = t.y;
-            }
 #pragma unroll
-            for (int i = 0; i < UN; i++) {
-                a[i][0] = fmaf(d[i], v.x, a[i][0]); a[i][1] = fmaf(d[i], v.y, a[i][1]);
-                a[i][2] = fmaf(d[i], v.z, a[i][2]); a[i][3] = fmaf(d[i], v.w, a[i][3]);
+                for (int i = 0; i < UN / 4; i++) {
+                    const float4 t = *reinterpret_cast<const float4 *>(pd + 4 * i);
+                    d[2 * i] = make_float2(t.x, t.y);
+                    d[2 * i + 1] = make_float2(t.z, t.w);
+                }
+            }
+            const float2 vx = make_float2(v.x, v.x), vy = make_float2(v.y, v.y), vz = make_float2(v.z, v.z),
+                         vw = make_float2(v.w, v.w);
+#pragma unroll
+            for (int i = 0; i < UN / 2; i++) {
+                a[i][0] = fma2(d[i], vx, a[i][0]); a[i][1] = fma2(d[i], vy, a[i][1]);
+                a[i][2] = fma2(d[i], vz, a[i][2]); a[i][3] = fma2(d[i], vw, a[i][3]);
             }
             pd += NR;
             pk += st;
@@ -490,10 +501,11 @@ __global__ void __launch_bounds__(NR == 16 ? 256 : 224) k_mlp_outer(const MlpWor
         for (int i = 0; i < UN; i++)
 #pragma unroll
             for (int j = 0; j < 4; j++) {
+                const float x = i & 1 ? a[i / 2][j].y : a[i / 2][j].x;
                 if (l1) {
-                    if (k + j < kMlpIn) put(kOffW1 + (n0 + un + i) * kMlpIn + k + j, a[i][j]);
+                    if (k + j < kMlpIn) put(kOffW1 + (n0 + un + i) * kMlpIn + k + j, x);
                 } else {
-                    put(kOffW2 + (n0 + un + i) * H + k + j, a[i][j]);
+                    put(kOffW2 + (n0 + un + i) * H + k + j, x);
                 }
             }
     } else if (tid >= 160) {
@@ -567,11 +579,12 @@ __device__ __forceinline__ void pack_param(const AdamArgs &o, int i, float p)
     }
 }
 
-// sum over the slots b (in order) of part[b][i]: added to grad[i], or (ADAM) the gradient of one
-// Adam step.  The last block: the loss, lsum's 32 partial sums per slot as the quad leaders and
-// warps of a tile add them, slots in order, into *loss (added to it unless ADAM).
-template <bool ADAM>
-__global__ void __launch_bounds__(128) k_mlp_reduce(const float *part, const double *lsum, int nb, double n,
+// sum over the slots b (in order) of part[b][i]: added to grad[i], or (kReduceAdam) the gradient of
+// one Adam step; kReduceGroups: so for each of ng consecutive groups of nb slots in turn.  The last block: the loss, lsum's 32 partial sums per slot as the quad leaders and
+// warps of a tile add them, slots in order, into *loss (added to it unless kReduceAdam).
+enum ReduceMode { kReduceAdd, kReduceGroups, kReduceAdam };
+template <ReduceMode MODE>
+__global__ void __launch_bounds__(128) k_mlp_reduce(const float *part, const double *lsum, int nb, int ng, double n,
                                                     float *grad, double *loss, const AdamArgs o)
 {
     grid_launch_dependents();
@@ -593,25 +606,43 @@ __global__ void __launch_bounds__(128) k_mlp_reduce(const float *part, const dou
         if (threadIdx.x == 0) {
             double l = 0.0;
             for (int b = 0; b < nb; b++) l += tile[b];
-            *loss = (ADAM ? 0.0 : *loss) + l;
+            *loss = (MODE == kReduceAdam ? 0.0 : *loss) + l;
         }
         return;
     }
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= kMlpParams) return;
-    const float *p = part + i;
-    float a = 0.f;
-    int b = 0;
-    for (; b + 16 <= nb; b += 16, p += 16 * kMlpParams) {
-        float v[16];
+    auto slots = [&](int k, int i) {  // group k's slots of parameter i, in order
+        const float *p = part + (int64_t)k * nb * kMlpParams + i;
+        float a = 0.f;
+        int b = 0;
+        for (; b + 16 <= nb; b += 16, p += 16 * kMlpParams) {
+            float v[16];
 #pragma unroll
-        for (int j = 0; j < 16; j++) v[j] = p[j * kMlpParams];
+            for (int j = 0; j < 16; j++) v[j] = p[j * kMlpParams];
 #pragma unroll
-        for (int j = 0; j < 16; j++) a += v[j];
+            for (int j = 0; j < 16; j++) a += v[j];
+        }
+        for (; b < nb; b++, p += kMlpParams) a += *p;
+        return a;
+    };
+    if constexpr (MODE == kReduceGroups) {
+        // 32 parameters per block, the groups' chains of additions over its four warps (one thread
+        // per parameter: 23 us for five groups of 109 slots, 13.6 us so)
+        __shared__ float gsum[4][32];
+        const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, i = blockIdx.x * 32 + lane;
+        float sum = i < kMlpParams ? grad[i] : 0.f;
+        for (int k0 = 0; k0 < ng; k0 += 4) {
+            gsum[w][lane] = k0 + w < ng && i < kMlpParams ? slots(k0 + w, i) : 0.f;
+            __syncthreads();
+            for (int k = k0; k < min(k0 + 4, ng); k++) sum += gsum[k - k0][lane];
+            __syncthreads();
+        }
+        if (w == 0 && i < kMlpParams) grad[i] = sum;
+    } else {
+        const int i = blockIdx.x * blockDim.x + threadIdx.x;
+        if (i >= kMlpParams) return;
+        if constexpr (MODE == kReduceAdam) pack_param(o, i, adam_param(o, i, 0.f + slots(0, i)));
+        else grad[i] += slots(0, i);
     }
-    for (; b < nb; b++, p += kMlpParams) a += *p;
-    if constexpr (ADAM) pack_param(o, i, adam_param(o, i, 0.f + a));
-    else grad[i] += a;
 }
 
 __global__ void k_mlp_pack(const float *m, uint16_t *w1, uint16_t *w2, float *b1, float *b2, float *w3, float *b3)
@@ -658,7 +689,7 @@ cudaError_t launch_outer(const MlpWork &w, int slots, bool first, cudaStream_t s
     return launch_after(k_mlp_outer<16>, dim3(4, slots), 256, smem_outer<16>(), s, true, w, first);
 }
 
-constexpr int kReduceBlocks = (kMlpParams + 127) / 128 + 1;
+constexpr int kReduceBlocks = (kMlpParams + 127) / 128 + 1, kGroupBlocks = (kMlpParams + 31) / 32 + 1;
 
 // Rows of a pass per round: every slot one tile.
 int64_t round_rows(int64_t n) { return std::min<int64_t>((n + kMlpTile - 1) / kMlpTile, kMlpMaxSlots) * kMlpTile; }
@@ -718,7 +749,7 @@ cudaError_t mlp_loss_grad(const MlpDev &net, const float *x, const float *t, int
     int nb = 0;
     cudaError_t e = sample_pass(net, x, t, nullptr, n, w, nb, s, false);
     if (e != cudaSuccess) return e;
-    return launch_after(k_mlp_reduce<false>, dim3(kReduceBlocks), 128, 0, s, true, w.part, w.lsum, nb, (double)n, grad, loss,
+    return launch_after(k_mlp_reduce<kReduceAdd>, dim3(kReduceBlocks), 128, 0, s, true, w.part, w.lsum, nb, 1, (double)n, grad, loss,
                   AdamArgs{});
 }
 
@@ -729,30 +760,57 @@ cudaError_t mlp_train_step(const MlpDev &net, const float *x, const float *t, co
     int nb = 0;
     cudaError_t e = sample_pass(net, x, t, idx, n, w, nb, s, dependent);
     if (e != cudaSuccess) return e;
-    return launch_after(k_mlp_reduce<true>, dim3(kReduceBlocks), 128, 0, s, true, w.part, w.lsum, nb, (double)n, nullptr,
+    return launch_after(k_mlp_reduce<kReduceAdam>, dim3(kReduceBlocks), 128, 0, s, true, w.part, w.lsum, nb, 1, (double)n, nullptr,
                   loss, adam_args(adam));
 }
 
-cudaError_t mlp_boundary_grad(const MlpDev &net, const BpttFields &f, const float *lm, const float *lm1,
-                              const float *lm2, float *grad, const MlpWork &w, cudaStream_t s)
+static MlpWork work_at(const MlpWork &w, int64_t row)
+{
+    MlpWork r = w;
+    r.xb += row * KXB; r.h1 += row * H; r.dz1 += row * H; r.dz2 += row * H; r.g2 += row * H; r.dy += row; r.err += row;
+    r.lsum = nullptr;
+    return r;
+}
+
+// Steps whose rows fit the work arrays together: one entry-parallel launch for all of them fills the
+// SMs and is paid once (109 tiles alone 13.7 us, five steps' 545 tiles 52 us: the tiles' 63 KB each
+// come from L2), and one reduction for all of them.
+int mlp_boundary_groups(int64_t nb)
+{
+    const int64_t tiles = (nb + kMlpTile - 1) / kMlpTile;
+    return (int)std::max<int64_t>(1, kMlpMaxSlots / std::max<int64_t>(tiles, 1));
+}
+
+cudaError_t mlp_boundary_rows(const MlpDev &net, const BpttFields &f, const float *lm, const float *lm1,
+                              const float *lm2, int group, const MlpWork &w, float *grad, cudaStream_t s)
 {
     if (f.nb <= 0) return cudaSuccess;
-    MlpWork ww = w;
-    ww.lsum = nullptr;
     const int64_t step = round_rows(f.nb);
-    const int nb = (int)(step / kMlpTile);
+    const bool rounds = step < f.nb;
+    const MlpWork ww = work_at(w, group * step);
     cudaError_t e = cudaSuccess;
     for (int64_t r0 = 0; r0 < f.nb && e == cudaSuccess; r0 += step) {
         const int64_t rows = round_rows(std::min(step, f.nb - r0));
         // three CTAs of 32 rows fit an SM
-        k_mlp_boundary<32><<<(unsigned)std::min<int64_t>(rows / 32, 152 * 3), 256, sizeof(RowSmem<32, true>), s>>>(
-            net, f, lm, lm1, lm2, ww, r0, rows);
-        e = cudaGetLastError();
-        if (e == cudaSuccess) e = launch_outer(ww, (int)(rows / kMlpTile), r0 == 0, s);
+        e = launch_after(k_mlp_boundary<32>, dim3((unsigned)std::min<int64_t>(rows / 32, 152 * 3)), 256,
+                         sizeof(RowSmem<32, true>), s, true, net, f, lm, lm1, lm2, ww, r0, rows);
+        if (e == cudaSuccess && rounds) e = launch_outer(ww, (int)(rows / kMlpTile), r0 == 0, s);
     }
+    if (e == cudaSuccess && rounds)
+        e = launch_after(k_mlp_reduce<kReduceAdd>, dim3(kReduceBlocks), 128, 0, s, true, w.part, (const double *)nullptr,
+                         (int)(step / kMlpTile), 1, 1.0, grad, (double *)nullptr, AdamArgs{});
+    return e;
+}
+
+cudaError_t mlp_boundary_params(int64_t nb, int n, float *grad, const MlpWork &w, cudaStream_t s)
+{
+    const int64_t step = round_rows(nb);
+    if (nb <= 0 || n <= 0 || step < nb) return cudaSuccess;  // (in rounds: already added)
+    const int tiles = (int)(step / kMlpTile);
+    cudaError_t e = launch_outer(work_at(w, 0), tiles * n, true, s);
     if (e != cudaSuccess) return e;
-    return launch_after(k_mlp_reduce<false>, dim3(kReduceBlocks), 128, 0, s, true, w.part, (const double *)nullptr, nb, 1.0,
-                  grad, (double *)nullptr, AdamArgs{});
+    return launch_after(k_mlp_reduce<kReduceGroups>, dim3(kGroupBlocks), 128, 0, s, true, w.part, (const double *)nullptr,
+                        tiles, n, 1.0, grad, (double *)nullptr, AdamArgs{});
 }
 
 cudaError_t mlp_adam(const MlpAdam &adam, const float *grad, cudaStream_t s)

@@ -81,11 +81,15 @@ struct BpttFields {
     const int64_t *nodes;       // boundary nodes (device layout), nb of them
     int64_t nb;
     const int *sidx;            // [n_int]: index in `nodes`, -1 elsewhere
-    float *dx;                  // [nb][81] feature gradient
+    const int64_t *shell;       // nodes within one of the boundary, n_shell of them
+    int64_t n_shell;
+    float *dx;                  // [81][dx_stride] feature gradient
+    int64_t dx_stride;
     float *a[3];                // adjoints of out^m, out^{m-1}, out^{m-2}
     float *v;                   // [n_int] work field
     const int64_t *roi;         // region of interest (device layout), n_roi nodes
     int n_roi;
+    const int *ridx;            // [n_int]: index in the region, -1 elsewhere (null: it lists a node twice)
 };
 // The stiffness operator of the stencil pass: 1-D table T[l][d + o] (direct form, diagonal
 // included), assembled weights by local index, g for the x, z and y terms.
@@ -95,12 +99,19 @@ struct BpttOperator {
     float wa[kMaxOrder];
     float g[3];
 };
-// Feature gradients gathered into A0, A1, A2.
-cudaError_t bptt_scatter(const BpttFields &f, cudaStream_t s);
-// Interior leapfrog adjoint (A0 -> A1, A2); a_mass = dt^2 / M.
-cudaError_t bptt_interior(const BpttFields &f, const BpttOperator &op, const float *a_mass, cudaStream_t s);
-// Loss over the region of interest at one step and its gradient into A0.
-cudaError_t bptt_loss(const BpttFields &f, const float *out, const float *ref, double *loss, cudaStream_t s);
+// Feature gradients gathered into A0, A1, A2, and v = a s A0 on interior nodes (a_mass = dt^2 / M).
+cudaError_t bptt_scatter(const BpttFields &f, const float *a_mass, cudaStream_t s);
+// Interior leapfrog adjoint (v, A0 -> A1, A2; A0 cleared); with next_out the loss gradient of that
+// level against next_ref is added to A1 (needs f.ridx).
+cudaError_t bptt_interior(const BpttFields &f, const BpttOperator &op, const float *next_out, const float *next_ref,
+                          cudaStream_t s);
+// Loss gradient of one level into A0.
+cudaError_t bptt_seed(const BpttFields &f, const float *out, const float *ref, cudaStream_t s);
+// Loss over the region of interest at every step: loss[m] of levels + m * stride against row m of ref.
+cudaError_t bptt_losses(const BpttFields &f, const float *levels, int64_t stride, const float *ref, int n_steps,
+                        double *loss, cudaStream_t s);
+// dst <- src, n floats (a multiple of 4), behind the preceding kernel of the stream.
+cudaError_t bptt_copy_level(const float *src, float *dst, int64_t n, cudaStream_t s);
 
 // bf16 conversion of the FP32 master weights into the device layout.
 cudaError_t mlp_pack(const float *master, uint16_t *w1, uint16_t *w2, float *b1, float *b2, float *w3, float *b3,
@@ -141,11 +152,16 @@ cudaError_t mlp_loss_grad(const MlpDev &net, const float *x, const float *t, int
 // preceding work of the stream is a step on the same network.
 cudaError_t mlp_train_step(const MlpDev &net, const float *x, const float *t, const int64_t *idx, int64_t n,
                            double *loss, const MlpAdam &adam, const MlpWork &w, cudaStream_t s, bool dependent);
-// One step of the adjoint of the time loop at the boundary nodes: features from the levels out^m,
-// out^{m-1}, out^{m-2}, output gradient from A0, parameter gradients added to grad, feature
-// gradients into f.dx.
-cudaError_t mlp_boundary_grad(const MlpDev &net, const BpttFields &f, const float *lm, const float *lm1,
-                              const float *lm2, float *grad, const MlpWork &w, cudaStream_t s);
+// The network in one step of the adjoint of the time loop, at the boundary nodes: features from the
+// levels out^m, out^{m-1}, out^{m-2}, output gradient from A0, feature gradients into f.dx, and the
+// rows' part of the parameter gradients into the work arrays' group `group` (the steps of one
+// mlp_boundary_params call).  Boxes of more boundary nodes than mlp_work_rows(nb) run in rounds and
+// add their parameter gradients to grad at once (mlp_boundary_groups returns 1).
+int mlp_boundary_groups(int64_t nb);
+cudaError_t mlp_boundary_rows(const MlpDev &net, const BpttFields &f, const float *lm, const float *lm1,
+                              const float *lm2, int group, const MlpWork &w, float *grad, cudaStream_t s);
+// Parameter gradients of groups 0..n-1 added to grad, group by group.
+cudaError_t mlp_boundary_params(int64_t nb, int n, float *grad, const MlpWork &w, cudaStream_t s);
 // One Adam step with a given gradient.
 cudaError_t mlp_adam(const MlpAdam &adam, const float *grad, cudaStream_t s);
 // Boundary correction: corr[i] = scale_i * net(features_i / scale_i) for the strip nodes.

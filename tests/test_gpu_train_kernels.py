@@ -76,3 +76,48 @@ def test_adjoint_over_two_rounds_of_boundary_nodes(semgb_lib, cuda_device):
         assert abs(fd - ad) <= 2e-2 * abs(fd), (fd, ad)
     for x in (abc, net, s, mesh):
         x.close()
+
+
+@pytest.mark.parametrize("twice", [False, True])
+def test_adjoint_step_groups_and_repeated_region_nodes(semgb_lib, cuda_device, twice):
+    """The adjoint sums the parameter gradients of several steps at once: on a 3^3 order-2 box (2 tiles
+    of boundary nodes, 304 steps per group) 310 steps take two groups, 304 exactly one, each against
+    central differences; and a region of interest that lists nodes twice counts them twice."""
+    semgb = semgb_lib
+    from semgb import workloads as W
+    ne, o, h, c = 3, 2, 10.0, 2000.0
+    for steps in (304, 310):
+        mesh = semgb.Mesh(ne, ne, ne, ne * h, ne * h, ne * h, o)
+        mesh.set_velocity(np.full(ne ** 3, c, np.float32))
+        s = semgb.Solver(mesh, W.cfl_dt(h, o, c))
+        s.set_kernel(semgb.KERNEL_STENCIL)
+        s.set_sponge(1, 0.1)
+        wav = np.exp(-((np.arange(steps) - (steps - 14)) / 4.0) ** 2)[None].astype(np.float32)  # late pulse
+        s.set_sources(np.array([1 + ne + ne * ne]), wav)
+        net = semgb.Mlp(3)
+        rng = np.random.default_rng(13)
+        p0 = (rng.standard_normal(M.N_PARAMS) * 0.02).astype(np.float32)
+        net.params = p0
+        abc = semgb.Abc(s, net, 0)
+        roi = np.arange(100, 200)
+        if twice:
+            roi = np.concatenate([roi, roi[::-1]])
+        ref = np.zeros((steps, len(roi)), np.float32)
+        loss, g = abc.bptt(roi, ref)
+        assert loss > 0 and np.all(np.isfinite(g))
+        if twice:
+            l1, g1 = abc.bptt(roi[:100], ref[:, :100])
+            assert abs(loss - 2 * l1) <= 1e-6 * loss and rel_l2(g, 2 * g1) < 1e-4
+        h1 = 64 * 81
+        fp32 = np.r_[np.arange(h1, h1 + 64), np.arange(h1 + 64 + 4096, len(p0))]
+        v = np.zeros_like(p0)
+        v[fp32] = rng.standard_normal(len(fp32)).astype(np.float32)
+        lp = []
+        for sign in (1.0, -1.0):
+            net.params = p0 + np.float32(sign * 1e-2) * v
+            lp.append(abc.bptt(roi, ref, grad=False)[0])
+        fd = (lp[0] - lp[1]) / 2e-2
+        ad = float(np.dot(g.astype(np.float64), v.astype(np.float64)))
+        assert abs(fd - ad) <= 2e-2 * abs(fd), (steps, fd, ad)
+        for x in (abc, net, s, mesh):
+            x.close()

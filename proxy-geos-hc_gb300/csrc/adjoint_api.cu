@@ -296,23 +296,46 @@ int sem_adjoint_backward(sem_adjoint *a, const float *residual, float *grad)
     // adjoint sources: residuals at the interior receiver nodes, newest step first, coefficient s a
     std::vector<int64_t> nodes;
     std::vector<float> coef, wav;
-    CUDA_TRY(cudaStreamSynchronize(f->stream));
+    std::vector<int> rows;  // receiver of each adjoint source
     for (int r = 0; r < a->nrec; r++) {
         const int64_t q = a->rec[r];
         const int64_t iy = q / (b.nxp * b.nz), rr = q - iy * b.nxp * b.nz, iz = rr / b.nxp, ix = rr - iz * b.nxp;
         if (ix == 0 || ix == b.nx - 1 || iy == 0 || iy == b.ny - 1 || iz == 0 || iz == b.nz - 1) continue;
-        float av = 0.f;
-        CUDA_TRY(cudaMemcpy(&av, f->d_a + q, 4, cudaMemcpyDeviceToHost));
-        const float s = a->sponge ? a->sx[ix] * a->sy[iy] * a->sz[iz] : 1.f;
         nodes.push_back(q);
-        coef.push_back(s * av);
-        for (int j = 0; j < N; j++) wav.push_back(residual[(size_t)(N - 1 - j) * a->nrec + r]);
+        coef.push_back(a->sponge ? a->sx[ix] * a->sy[iy] * a->sz[iz] : 1.f);
+        rows.push_back(r);
+    }
+    const size_t ns = nodes.size();
+    if (ns > 0) {
+        // a = dt^2/M at the source nodes, gathered in one launch
+        std::vector<float> av(ns);
+        int64_t *d_nodes = nullptr;
+        float *d_av = nullptr;
+        cudaError_t e = dalloc(&d_nodes, ns);
+        if (e == cudaSuccess) e = dalloc(&d_av, ns);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(d_nodes, nodes.data(), ns * 8, cudaMemcpyHostToDevice, f->stream);
+        if (e == cudaSuccess) e = launch_gather_nodes(f->d_a, d_nodes, (int)ns, d_av, f->stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(av.data(), d_av, ns * 4, cudaMemcpyDeviceToHost, f->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(f->stream);
+        dfree(d_nodes);
+        dfree(d_av);
+        CUDA_TRY(e);
+        wav.resize(ns * N);
+        for (size_t k = 0; k < ns; k++) {
+            coef[k] *= av[k];
+            for (int j = 0; j < N; j++) wav[k * N + j] = residual[(size_t)(N - 1 - j) * a->nrec + rows[k]];
+        }
     }
     if ((rc = solver_set_raw_sources(g, (int)nodes.size(), nodes.data(), coef.data(), wav.data(), N)) != SEM_OK)
         return rc;
     if ((rc = sem_solver_reset(g)) != SEM_OK) return rc;
-    if ((rc = solver_prepare(g, N)) != SEM_OK) return rc;
     if ((rc = solver_prepare(f, 0)) != SEM_OK) return rc;
+    if (g->a_version != f->a_version) {
+        // the same mesh, model and dt: the forward run's dt^2/M
+        CUDA_TRY(cudaMemcpyAsync(g->d_a, f->d_a, lv * 4, cudaMemcpyDeviceToDevice, f->stream));
+        g->a_version = f->a_version;
+    }
+    if ((rc = solver_prepare(g, N)) != SEM_OK) return rc;
     CUDA_TRY(cudaMemsetAsync(a->d_grad, 0, lv * 4, f->stream));
     if (a->seg_gen[0] != f->graph_gen || a->seg_gen[1] != g->graph_gen) {
         destroy_seg_graphs(a);

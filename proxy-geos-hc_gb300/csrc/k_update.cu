@@ -195,29 +195,80 @@ __global__ void k_mass_ref(float *m, const float *vel, int ex, int ey, int ez, i
         }
 }
 
+// (float)(n / d), the double quotient rounded to float, given x = 1/d to about 2^-45: one Newton
+// correction gives the quotient to within an ulp of double, which rounds to the same float unless it
+// lies within a few ulps of a midpoint between floats or outside the normal range; those take the
+// division.  Double-precision operations are what the kernel below spends its time on (two lanes per SM
+// and clock): three here against about ten.  (For dt^2/M, whose divisor differs per node, a float
+// reciprocal and a Newton step measured slower than the division: 1.3 against 0.9 ms.)
+__device__ __forceinline__ float quotient_float(const double n, const double d, const double x)
+{
+    if (n == 0.0) return (float)n;
+    double q = n * x;
+    q = fma(fma(-d, q, n), x, q);
+    const int low = (int)(__double_as_longlong(q) & 0x1fffffff) - 0x10000000;
+    const double m = fabs(q);
+    if (!(m >= 1.1754943508222875e-38 && m <= 1e38) || (low >= -4 && low <= 4)) q = n / d;
+    return (float)q;
+}
+
+// Products of the local weights and detJ, ((w_x w_z) w_y) detJ, by local index (lx + o (lz + o ly)).
+__device__ __forceinline__ void weight_table(double *t, const double *w, const int o, const double detJ)
+{
+    for (int i = threadIdx.x; i < o * o * o; i += blockDim.x)
+        t[i] = w[i % o] * w[i / o % o] * w[i / (o * o)] * detJ;
+}
+
+constexpr int kScaleRows = 4;  // rows along z per block
+constexpr int kMaxCube = 125;
+
 // g_i <- g_i / m_i with m_i the node's squared slowness, recovered from the stored
 // a_i = dt^2 / (m_i W_i) and the geometric mass W_i (quadrature weight x detJ x adjacent elements),
-// so it holds for element-velocity and node-slowness models alike.
-__global__ void k_grad_scale(float *g, const float *a, int ex, int ey, int ez, int order, int64_t nxp,
-                             const double *w, double detJ, double dt2)
+// so it holds for element-velocity and node-slowness models alike.  Grid: x-blocks
+// of a row by kScaleRows rows along z by y (0.43 ms on 24.1 M nodes; 1.46 ms with three 64-bit divisions
+// of indices and a double division per node).
+__global__ void __launch_bounds__(128) k_grad_scale(float *g, const float *a, int ex, int ey, int ez, int order, int nxp,
+                                                    const double *w, double detJ, double dt2, double inv_dt2)
 {
-    const int64_t nx = (int64_t)ex * order + 1, ny = (int64_t)ey * order + 1,
-                  nz = (int64_t)ez * order + 1, n = nxp * ny * nz;
-    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n;
-         q += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t iy = q / (nxp * nz), r = q - iy * nxp * nz, iz = r / nxp, ix = r - iz * nxp;
-        if (ix >= nx) {
-            g[q] = 0.f;
-            continue;
-        }
-        const double wq = w[ix % order] * w[iz % order] * w[iy % order];
-        int x0, x1, z0, z1, y0, y1;
-        adj_range((int)ix, order, ex, x0, x1);
-        adj_range((int)iz, order, ez, z0, z1);
-        adj_range((int)iy, order, ey, y0, y1);
-        const double W = wq * detJ * (double)((x1 - x0 + 1) * (z1 - z0 + 1) * (y1 - y0 + 1));
-        g[q] = (float)((double)g[q] * (double)a[q] * W / dt2);
-    }
+    __shared__ double wt[kMaxCube];
+    weight_table(wt, w, order, detJ);
+    __syncthreads();
+    const int nx = ex * order + 1, ny = ey * order + 1, nz = ez * order + 1;
+    const int ix = blockIdx.x * blockDim.x + threadIdx.x;
+    if (ix >= nxp) return;
+    int x0 = 0, x1 = 0;
+    if (ix < nx) adj_range(ix, order, ex, x0, x1);
+    const int lx = ix % order;
+    for (int iy = blockIdx.z; iy < ny; iy += gridDim.z)
+        for (int zb = blockIdx.y * kScaleRows; zb < nz; zb += gridDim.y * kScaleRows)
+#pragma unroll
+            for (int r = 0; r < kScaleRows; r++) {
+                const int iz = zb + r;
+                if (iz >= nz) break;
+                const int64_t q = ix + (int64_t)nxp * (iz + (int64_t)nz * iy);
+                if (ix >= nx) {
+                    g[q] = 0.f;
+                    continue;
+                }
+                int z0, z1, y0, y1;
+                adj_range(iz, order, ez, z0, z1);
+                adj_range(iy, order, ey, y0, y1);
+                const double W = wt[lx + order * (iz % order + order * (iy % order))] *
+                                 (double)((x1 - x0 + 1) * (z1 - z0 + 1) * (y1 - y0 + 1));
+                g[q] = quotient_float((double)g[q] * (double)a[q] * W, dt2, inv_dt2);
+            }
+}
+
+// out[i] = a[nodes[i]]
+__global__ void k_gather_nodes(const float *a, const int64_t *nodes, int n, float *out)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = a[nodes[i]];
+}
+
+dim3 scale_grid(int64_t nxp, int64_t nz, int64_t ny)
+{
+    return dim3((unsigned)((nxp + 127) / 128), (unsigned)std::min<int64_t>((nz + kScaleRows - 1) / kScaleRows, 65535),
+                (unsigned)std::min<int64_t>(ny, 65535));
 }
 
 }  // namespace
@@ -225,7 +276,15 @@ __global__ void k_grad_scale(float *g, const float *a, int ex, int ey, int ez, i
 cudaError_t launch_grad_scale(float *g, const float *a, int ex, int ey, int ez, int order, int64_t nxp,
                               const double *w_dev, double detJ, double dt2, cudaStream_t s)
 {
-    k_grad_scale<<<152 * 16, 256, 0, s>>>(g, a, ex, ey, ez, order, nxp, w_dev, detJ, dt2);
+    const int64_t ny = (int64_t)ey * order + 1, nz = (int64_t)ez * order + 1;
+    k_grad_scale<<<scale_grid(nxp, nz, ny), 128, 0, s>>>(g, a, ex, ey, ez, order, (int)nxp, w_dev, detJ, dt2, 1.0 / dt2);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_gather_nodes(const float *a, const int64_t *nodes, int n, float *out, cudaStream_t s)
+{
+    if (n <= 0) return cudaSuccess;
+    k_gather_nodes<<<std::min((n + 255) / 256, 152), 256, 0, s>>>(a, nodes, n, out);
     return cudaGetLastError();
 }
 

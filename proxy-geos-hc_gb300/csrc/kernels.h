@@ -112,6 +112,8 @@ cudaError_t launch_connectivity(int32_t *conn, int ex, int ey, int ez, int order
 // Gradient with respect to the nodal mass parameter -> with respect to squared slowness: g /= m.
 cudaError_t launch_grad_scale(float *g, const float *a, int ex, int ey, int ez, int order, int64_t nxp,
                               const double *w_dev, double detJ, double dt2, cudaStream_t s);
+// out[i] = a[nodes[i]]
+cudaError_t launch_gather_nodes(const float *a, const int64_t *nodes, int n, float *out, cudaStream_t s);
 // a_i = dt^2 / M_i from per-element velocity (vel) or per-node squared slowness (slow2, device
 // layout); zero on padding nodes.
 cudaError_t launch_mass(float *a, const float *vel, const float *slow2, int ex, int ey, int ez,

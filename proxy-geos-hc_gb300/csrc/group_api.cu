@@ -135,7 +135,8 @@ int capture(sem_group *g, int parity)
 // resident CTA slots, each on the least loaded one (a member's CTAs all have the same work, so
 // they go in whole rounds over the slots, the remainder on the least loaded); a CTA's work is
 // its planes plus the 2o planes it reads before its first output.
-std::vector<int> group_chunks(const sem_group *g, int64_t resident)
+// far: whether the members leave out the tiles of far boundary nodes alone (StencilBox), chosen with L.
+std::vector<int> group_chunks(const sem_group *g, int64_t resident, bool &far)
 {
     const size_t n = g->members.size();
     int64_t ny_max = 1;
@@ -144,17 +145,25 @@ std::vector<int> group_chunks(const sem_group *g, int64_t resident)
     int64_t best_l = ny_max;
     std::vector<std::pair<int64_t, int64_t>> jobs;  // (CTA work in planes, CTA count)
     std::vector<double> load((size_t)std::max<int64_t>(resident, 1));
-    for (int64_t L = 1; L <= ny_max; L++) {
+    far = false;
+    for (int64_t k = 2; k < 2 * ny_max + 2; k++) {
+        const int64_t L = k / 2;
+        const bool fe = k & 1;
         jobs.clear();
         for (const sem_solver *s : g->members) {
             const Box &b = s->mesh->box;
             int tx = 0, tz = 0, hx = 0, th = 0;  // the member's own tile shape
             semgb::stencil_tile_dims(b.order, s->stencil->shape, tx, tz, hx, th);
-            const int64_t cols = ((b.nx + tx - 1) / tx) * ((b.nz + tz - 1) / tz);
+            const int64_t cols = semgb::stencil_tiles(b.nx, tx, fe) * semgb::stencil_tiles(b.nz, tz, fe);
             const int64_t c = (b.ny + L - 1) / L, chunk = (b.ny + c - 1) / c;
-            jobs.push_back({chunk + 2 * b.order, cols * c});
+            const bool edges = fe && ((b.nx - 1) % tx == 0 || (b.nz - 1) % tz == 0);
+            jobs.push_back({chunk + 2 * b.order + (edges ? semgb::kFarEdgeCost : 0), cols * c});
         }
         std::sort(jobs.begin(), jobs.end(), [](const auto &x, const auto &y) { return x.first > y.first; });
+        // no schedule beats the longest CTA or the average load: most lengths need no placing
+        double total = 0;
+        for (const auto &jb : jobs) total += (double)jb.first * (double)jb.second;
+        if (std::max((double)jobs.front().first, total / (double)load.size()) >= best - 1e-9) continue;
         std::fill(load.begin(), load.end(), 0.0);  // kept in ascending order
         const int64_t R = (int64_t)load.size();
         for (const auto &jb : jobs) {
@@ -166,7 +175,7 @@ std::vector<int> group_chunks(const sem_group *g, int64_t resident)
             std::inplace_merge(load.begin(), load.begin() + rem, load.end());
         }
         const double makespan = load.back();
-        if (makespan < best - 1e-9) { best = makespan; best_l = L; }
+        if (makespan < best - 1e-9) { best = makespan; best_l = L; far = fe; }
     }
     std::vector<int> out(n);
     for (size_t i = 0; i < n; i++) {
@@ -252,7 +261,8 @@ int build_one_launch(sem_group *g)
     CUDA_TRY(cudaGetDevice(&dev));
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int per_sm = std::max(1, semgb::group_blocks_per_sm(max_order));
-    const std::vector<int> chunks = group_chunks(g, (int64_t)sms * per_sm);
+    bool far = false;
+    const std::vector<int> chunks = group_chunks(g, (int64_t)sms * per_sm, far);
     for (auto &t : g->tabs) semgb::stencil_tables_free(t);
     g->tabs.assign(n, nullptr);
     if (g->ones.size() != n) g->ones.assign(n, nullptr);
@@ -260,7 +270,7 @@ int build_one_launch(sem_group *g)
         sem_solver *s = g->members[i];
         // tables of the member's own tile shape over its levels, with the group's chunking
         StencilTables *t = nullptr;
-        if (semgb::stencil_tables_create(s->mesh->box, s->mesh->gll, s->mesh->geo, 1, &t, s->stencil->shape) != 0)
+        if (semgb::stencil_tables_create(s->mesh->box, s->mesh->gll, s->mesh->geo, 1, &t, s->stencil->shape, far) != 0)
             return sem_fail(SEM_ERR_CUDA, "stencil tables");
         g->tabs[i] = t;
         if (semgb::stencil_bind(*t, s->d_p[0], s->d_p[1], s->d_a) != 0)

@@ -58,26 +58,35 @@ __global__ void __launch_bounds__(kGroupThreads, kGroupMinBlocks)
     k_group(const GroupMember *__restrict__ mem, const int *__restrict__ cta_member, int k, int step_off, int inject)
 {
     const GroupMember &g = mem[__ldg(cta_member + blockIdx.x)];
-    const StencilTables &t = g.t;
-    const int ci = g.cur0 ^ k;
+    // the member's box and arguments in shared memory: every use in the pass reads them from there instead
+    // of global memory (through the references they are read again after each barrier or copy)
+    __shared__ alignas(16) int s_box[sizeof(StencilBox) / 4], s_args[sizeof(StencilArgs) / 4];
+    static_assert(sizeof(StencilBox) % 4 == 0 && sizeof(StencilArgs) % 4 == 0 && sizeof(StencilBox) <= 4 * kGroupThreads &&
+                      sizeof(StencilArgs) <= 4 * kGroupThreads, "one word per thread");
+    const StencilBox *gbox = &g.t;
+    if (threadIdx.x < sizeof(StencilBox) / 4) s_box[threadIdx.x] = reinterpret_cast<const int *>(gbox)[threadIdx.x];
+    if (threadIdx.x < sizeof(StencilArgs) / 4) s_args[threadIdx.x] = reinterpret_cast<const int *>(&g.a[k])[threadIdx.x];
+    const int ci = g.cur0 ^ k, order = g.order, shape = g.t.shape;
     const int local = (int)blockIdx.x - g.cta0;  // CTA within the member: x-tile fastest, then z, then chunk
+    __syncthreads();
+    const StencilBox &t = *reinterpret_cast<const StencilBox *>(s_box);
+    const StencilArgs &a = *reinterpret_cast<const StencilArgs *>(s_args);
     const int bx = local % t.grid[0], rz = local / t.grid[0];
     const int bz = rz % t.grid[1], chunk = rz / t.grid[1];
-    const CUtensorMap *rmap = &t.lv[ci].tile, *wmap = &t.lv[ci].win, *pmap = &t.lv[1 - ci].tile, *amap = &t.amap;
+    const CUtensorMap *rmap = &g.t.lv[ci].tile, *wmap = &g.t.lv[ci].win, *pmap = &g.t.lv[1 - ci].tile, *amap = &g.t.amap;
     if (threadIdx.x == 0) {
         tensormap_acquire(rmap);
         tensormap_acquire(wmap);
         tensormap_acquire(pmap);
         tensormap_acquire(amap);
     }
-    const StencilArgs &a = g.a[k];
     const NoClassTable none{};
-    switch (g.order) {
+    switch (order) {
     case 1: stencil_cta<1, true, STENCIL_PLAIN, true, false, false, true>(rmap, wmap, pmap, amap, t, a, none, 0, bx, bz, chunk, step_off, inject != 0); break;
     case 2: stencil_cta<2, true, STENCIL_PLAIN, true, false, false, true>(rmap, wmap, pmap, amap, t, a, none, 0, bx, bz, chunk, step_off, inject != 0); break;
     case 3: stencil_cta<3, true, STENCIL_PLAIN, true, false, false, true>(rmap, wmap, pmap, amap, t, a, none, 0, bx, bz, chunk, step_off, inject != 0); break;
     default:
-        if (t.shape == kTileSquare)
+        if (shape == kTileSquare)
             stencil_cta<4, true, STENCIL_PLAIN, true, false, false, true, kSquareRW>(rmap, wmap, pmap, amap, t, a, none, 0,
                                                                                      bx, bz, chunk, step_off, inject != 0);
         else

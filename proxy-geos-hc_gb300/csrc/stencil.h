@@ -48,6 +48,11 @@ struct StencilBox {
     int grid[3] = {0, 0, 0};  // tiles along x, z and y-chunks (launch: x * z * nshot CTAs by chunks)
     int nshot = 1;            // shots stacked along y in the levels (many-shot form)
     int ychunk = 0;           // planes per CTA
+    // 1: the last node along x (z) has no tile, the others fill whole tiles (see far_edges)
+    int far_x = 0, far_z = 0;
+    // Planes of a chunk divided among `parts` CTAs: first plane of part k, and the part of a plane.
+    __host__ __device__ static int part_begin(int planes, int parts, int k) { return (int)(((int64_t)planes * k + parts - 1) / parts); }
+    __host__ __device__ static int part_of(int planes, int parts, int y) { return (int)((int64_t)y * parts / planes); }
 };
 
 struct StencilTables : StencilBox {
@@ -130,12 +135,24 @@ cudaError_t launch_group_source(const GroupMember *members, int n_members, int k
 cudaError_t launch_group_pass(const GroupMember *members, const int *cta_member, int n_ctas, int max_order, int k,
                               int step_off, bool inject, cudaStream_t s);
 
+// Tiles of `tile` nodes along an axis of n; far: where n is whole tiles plus one node, that node,
+// always on the boundary, gets none (the pass's far_edges).
+inline int64_t stencil_tiles(int64_t n, int tile, bool far)
+{
+    return far && (n - 1) % tile == 0 ? (n - 1) / tile : (n + tile - 1) / tile;
+}
+// Planes of a CTA's march that damping its share of the far edges is taken to cost (a few dependent
+// memory latencies before the march): small boxes, whose CTAs are all resident at once, keep the extra
+// tiles (40^3 elements of order 2: 4.7 us per step with them, 4.85 without; a group of 32 boxes of 8 to
+// 24 elements 34.1 against 42.7), larger ones drop them.
+constexpr int kFarEdgeCost = 6;
 // Tables and tiling for a box (no device buffers yet).  Returns 0 or a cudaError_t.
 // nshot > 1: the many-shot form, levels holding nshot fields one after another (traces
 // [step][receiver][shot]); dt^2/M and the sponge are shared.
 // shape: kTileDefault, kTileSquare (order 4, one shot; otherwise the default) or -1 to choose
+// far: 1 (0) to leave out (keep) tiles of far boundary nodes alone, -1 to choose
 int stencil_tables_create(const Box &b, const Gll &g, const Geometry &geo, int nshot, StencilTables **out,
-                          int shape = -1);
+                          int shape = -1, int far = -1);
 // tile of a shape: nodes along x and z, x halo, threads per CTA
 void stencil_tile_dims(int order, int shape, int &tx, int &tz, int &hx, int &threads);
 // Describe the solver's two pressure buffers and its dt^2/M buffer with tensor maps.

@@ -325,6 +325,62 @@ template <int O, bool REF>
 using ClassParam = typename std::conditional<REF, ClassTable<O>, NoClassTable>::type;
 
 
+// Far boundary nodes without a tile: where the mesh is whole tiles plus its last node along an axis and
+// the plan says so (StencilBox::far_x, far_z), that node -- always on the boundary, where a step only damps the stored
+// previous level twice -- gets no tile of its own (stencil_tiles).  A chunk's planes of the far row
+// over a column of tiles are divided among that column's CTAs (along z), those of the far column among
+// the CTAs along x, and damped while a CTA's first copies are on their way.  A tile for one row cost
+// 40^3 elements of order 4 a tenth of the pass's CTAs, 96^3 of order 3 a sixth; left to the last tile's
+// CTA alone the rows took longer than they saved (200^3 of order 4: 1533 against 1392 us).
+// Not inlined: in line its index arithmetic moved the march's code, whose time follows such moves by
+// up to 2 % (200^3 of order 4: 1344 against 1376 us with the same work).
+struct FarEdges {
+    float *p;                    // stored previous level (of the shot), new level out
+    const float *sx, *sy, *sz;
+    int64_t nxp;
+    int nx, nz, tx, tz, gx, gz;  // nodes, tile and tiles along x and z
+    int fx, fz;
+};
+__device__ __noinline__ void far_edges(const FarEdges f, const int bx, const int bz, const int yb, const int planes)
+{
+    const bool fx = f.fx != 0, fz = f.fz != 0;
+    const int x0 = bx * f.tx, z0 = bz * f.tz, step = (int)blockDim.x;
+    if (fz) {
+        // row nz - 1 over the tile's columns (and the corner), four nodes at a time; columns past the
+        // mesh are padding and stay zero
+        const int w = (min(x0 + f.tx + (fx && bx == f.gx - 1 ? 1 : 0), f.nx) - x0 + 3) / 4;
+        const int y0 = StencilBox::part_begin(planes, f.gz, bz);
+        const int count = (StencilBox::part_begin(planes, f.gz, bz + 1) - y0) * w;
+        const float szv = __ldg(f.sz + f.nz - 1);
+        for (int i = (int)threadIdx.x; i < count; i += step) {
+            const int y = yb + y0 + i / w, x = x0 + i % w * 4;
+            float4 *q = reinterpret_cast<float4 *>(f.p + x + f.nxp * (f.nz - 1 + f.nz * (int64_t)y));
+            const float4 v = *q;
+            const float syv = __ldg(f.sy + y);
+            float r[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const float sv = (x + k < f.nx ? __ldg(f.sx + x + k) * szv : 0.f) * syv;
+                r[k] = sv * (sv * r[k]);
+            }
+            *q = make_float4(r[0], r[1], r[2], r[3]);
+        }
+    }
+    if (fx) {
+        // column nx - 1 over the tile's rows
+        const int h = min(f.tz, f.nz - z0);
+        const int y0 = StencilBox::part_begin(planes, f.gx, bx);
+        const int count = (StencilBox::part_begin(planes, f.gx, bx + 1) - y0) * h;
+        const float sxv = __ldg(f.sx + f.nx - 1);
+        for (int i = (int)threadIdx.x; i < count; i += step) {
+            const int y = yb + y0 + i / h, z = z0 + i % h;
+            float *q = f.p + f.nx - 1 + f.nxp * (z + f.nz * (int64_t)y);
+            const float sv = (sxv * __ldg(f.sz + z)) * __ldg(f.sy + y);
+            *q = sv * (sv * *q);
+        }
+    }
+}
+
 // REF: the reference-rounding operator -- every coefficient from the node-class table `ct`, one
 // accumulation per node over the x-, z- and y-terms (direct form only).
 //
@@ -423,6 +479,11 @@ __device__ __forceinline__ void stencil_cta(const CUtensorMap *rmap, const CUten
     const int64_t group_stride = (int64_t)GR * nxp;
 
     grid_dependency_wait();
+    if (SPONGE && (t.far_x | t.far_z))  // (no sponge: the stored level stays as it is)
+        far_edges(FarEdges{a.prev + (MULTI ? (int64_t)shot * t.shot_stride : 0), a.sx, a.sy, a.sz, t.nxp, nx, nz, TX, TZ,
+                           t.grid[0], t.grid[1],
+                           t.far_x, t.far_z},
+                  bx, bz, yb, ye - yb);
     bool ok = true;
     for (int p = yb - O; p < yb + O; p++) {
         const int i = p - yb + O;  // < 2O < R: first fill of each of these slots
@@ -682,6 +743,7 @@ __device__ __forceinline__ void stencil_cta(const CUtensorMap *rmap, const CUten
                 const int64_t q = a.src.node[shot];
                 if (threadIdx.x == 0 && q >= 0) {
                     const int64_t plane = t.nxp * t.nz, y = q / plane, r = q - y * plane, zz = r / t.nxp, x = r - zz * t.nxp;
+                    // (a source node is the first of its element: never on a far edge)
                     if (x / TX == bx && zz / TZ == bz && y / t.ychunk == chunk)
                         lvl[q] += a.src.coef[shot] * a.src.wavelet[(int64_t)shot * a.src.nsamples + n];
                 }

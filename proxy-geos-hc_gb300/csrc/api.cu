@@ -151,6 +151,9 @@ cudaError_t field_from_host(float *dst, const float *src, int64_t nx, int64_t nx
     return e != cudaSuccess ? e : es;
 }
 
+// Largest receiver read of sem_solver_step_host that goes through the solver's pinned buffer (64 KB).
+static constexpr int64_t kPinFloats = 1 << 14;
+
 static int resolved_kernel(const sem_solver *s)
 {
     return s->kernel == SEM_KERNEL_AUTO ? SEM_KERNEL_STENCIL : s->kernel;
@@ -508,6 +511,7 @@ int sem_solver_destroy(sem_solver *s)
     dfree(s->d_ctr);
     dfree(s->d_status);
     dfree(s->d_upd_rec_off);
+    if (s->pin) cudaFreeHost(s->pin);
     if (s->own_stream && s->stream) cudaStreamDestroy(s->stream);
     delete s;
     return SEM_OK;
@@ -876,8 +880,12 @@ cudaError_t solver_enqueue_step(sem_solver *s, int c, cudaEvent_t *ev, const Ste
     const SourceTable src = solver_sources(s);
     if (ev) cudaEventRecord(ev[0], s->stream);
     if (x.advance > 0)
-        if ((e = launch_source(SourceArgs{s->d_p[c], src, s->d_ctr, x.advance}, s->stream, x.after)) != cudaSuccess)
-            return e;
+    {
+        const SourceArgs sa{s->d_p[c], src, s->d_ctr, x.advance};
+        e = x.samples ? launch_source_samples(sa, *x.samples, s->d_wavelet, s->stream)
+                      : launch_source(sa, s->stream, x.after);
+        if (e != cudaSuccess) return e;
+    }
     if (ev) cudaEventRecord(ev[1], s->stream);
     if (resolved_kernel(s) == SEM_KERNEL_ELEMENT) {
         if (x.mode != STENCIL_PLAIN || x.advance != 1 || x.inject) return cudaErrorInvalidValue;  // stencil pass only
@@ -1007,22 +1015,51 @@ int sem_solver_step_host(sem_solver *s, int n_steps, const float *wavelet_sample
     if (n_steps < 0) return fail(SEM_ERR_ARG, "n_steps must be >= 0");
     if (n_steps == 0) return SEM_OK;
     const int64_t n0 = s->steps_done;
+    HostSamples h{};
     if (wavelet_samples && s->nsrc > 0) {
         if (n0 + n_steps > s->nsamples)
             return fail(SEM_ERR_ARG, "wavelet storage shorter than the steps requested");
-        // host [n_steps][nsrc] -> device [nsrc][nsamples] columns n0..n0+n_steps-1
-        for (int k = 0; k < s->nsrc; k++)
-            CUDA_TRY(cudaMemcpy2DAsync(s->d_wavelet + (size_t)k * s->nsamples + n0, sizeof(float),
-                                       wavelet_samples + k, (size_t)s->nsrc * sizeof(float),
-                                       sizeof(float), n_steps, cudaMemcpyHostToDevice, s->stream));
+        if (n_steps == 1 && s->nsrc <= kMaxHostSamples) {
+            // one step's samples travel with the source launch
+            h.n = s->nsrc;
+            std::copy(wavelet_samples, wavelet_samples + s->nsrc, h.v);
+        } else {
+            // host [n_steps][nsrc] -> device [nsrc][nsamples] columns n0..n0+n_steps-1
+            for (int k = 0; k < s->nsrc; k++)
+                CUDA_TRY(cudaMemcpy2DAsync(s->d_wavelet + (size_t)k * s->nsamples + n0, sizeof(float),
+                                           wavelet_samples + k, (size_t)s->nsrc * sizeof(float),
+                                           sizeof(float), n_steps, cudaMemcpyHostToDevice, s->stream));
+        }
     }
-    int rc = sem_solver_step(s, n_steps);
-    if (rc) return rc;
-    if (traces_out && s->nrec > 0)
-        CUDA_TRY(cudaMemcpyAsync(traces_out, s->d_traces + (size_t)n0 * s->nrec,
-                                 (size_t)n_steps * s->nrec * sizeof(float), cudaMemcpyDeviceToHost,
-                                 s->stream));
+    if (h.n > 0) {
+        int rc = solver_prepare(s, 1);
+        if (rc) return rc;
+        StepExtra x;
+        x.samples = &h;
+        CUDA_TRY(solver_enqueue_step(s, s->cur, nullptr, &x));
+        s->cur ^= 1;
+        s->steps_done++;
+    } else {
+        int rc = sem_solver_step(s, n_steps);
+        if (rc) return rc;
+    }
+    const int64_t nt = (int64_t)n_steps * s->nrec;
+    const float *rows = nt > 0 ? s->d_traces + (size_t)n0 * s->nrec : nullptr;
+    if (traces_out && nt > 0 && nt <= kPinFloats && !s->pin) {
+        if (cudaHostAlloc(reinterpret_cast<void **>(&s->pin), kPinFloats * 4, cudaHostAllocMapped) != cudaSuccess ||
+            cudaHostGetDevicePointer(reinterpret_cast<void **>(&s->d_pin), s->pin, 0) != cudaSuccess) {
+            cudaGetLastError();
+            if (s->pin) cudaFreeHost(s->pin);
+            s->pin = nullptr;  // the copy below serves
+        }
+    }
+    const bool pinned = traces_out && nt > 0 && nt <= kPinFloats && s->pin;
+    if (pinned)  // written by the device: a copy into pageable memory is staged by the driver
+        CUDA_TRY(launch_rows_out(rows, s->d_pin, (int)nt, s->stream, n_steps % kGraphSteps != 0));
+    else if (traces_out && nt > 0)
+        CUDA_TRY(cudaMemcpyAsync(traces_out, rows, (size_t)nt * sizeof(float), cudaMemcpyDeviceToHost, s->stream));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
+    if (pinned) std::copy(s->pin, s->pin + nt, traces_out);
     return SEM_OK;
     GUARD_END
 }
@@ -1143,11 +1180,21 @@ int sem_solver_reset(sem_solver *s)
     if (!s) return fail(SEM_ERR_ARG, "NULL solver");
     // on the solver's own stream, which does not wait for the default stream: a step enqueued
     // after this call starts from the zeroed levels and step counter
-    for (auto p : s->d_p) CUDA_TRY(cudaMemsetAsync(p, 0, s->n_int * 4, s->stream));
-    if (s->d_y) CUDA_TRY(cudaMemsetAsync(s->d_y, 0, s->n_int * 4, s->stream));
-    CUDA_TRY(cudaMemsetAsync(s->d_ctr, 0, 8, s->stream));
-    CUDA_TRY(cudaMemsetAsync(s->d_status, 0, 4, s->stream));
-    if (s->d_traces) CUDA_TRY(cudaMemsetAsync(s->d_traces, 0, (size_t)s->trace_cap * s->nrec * 4, s->stream));
+    const int64_t nt = s->d_traces ? s->trace_cap * s->nrec : 0;
+    ZeroArgs z{{s->d_p[0], s->d_p[1], s->d_y, s->d_traces},
+               {s->n_int, s->n_int, s->d_y ? s->n_int : 0, nt},
+               {s->d_ctr, s->d_status},
+               {2, 1}};
+    // One launch costs the host 2.3 us and five fills 5.5; reset and wait, fills -> launch: order 2,
+    // 12^3 elements 26 -> 19 us, order 4: 31^3 28 -> 21, 80^3 (33 M nodes) 65 -> 61.  The fills write
+    // large levels faster (order 4, 120^3, 111 M nodes: 148 us against 160; 200^3: 572 against 663).
+    if (s->n_int + nt > (int64_t(1) << 26)) {
+        for (int k = 0; k < 4; k++) {
+            if (z.n[k] > 0) CUDA_TRY(cudaMemsetAsync(z.f[k], 0, (size_t)z.n[k] * 4, s->stream));
+            z.n[k] = 0;
+        }
+    }
+    CUDA_TRY(launch_zero(z, s->stream));
     s->steps_done = 0;
     s->traces_checked = 0;
     s->cur = 0;

@@ -33,6 +33,47 @@ __global__ void k_source(const SourceArgs a)
     }
 }
 
+// k_source on samples handed over by value.  A step streamed from the host costs latency: a 2-D copy
+// of one column of the wavelets from pageable memory, the launches and a copy back were 36 us a step
+// (12^3 elements, order 2, 16 receivers); samples by value 33, with the rows written by k_rows_out 28.
+__global__ void k_source_samples(const SourceArgs a, const HostSamples h, float *wavelet)
+{
+    grid_launch_dependents();  // the pass waits for this launch before it reads anything
+    const int n = a.ctr[0];
+    if (n < a.t.nsamples && (int)threadIdx.x < h.n) wavelet[(int64_t)threadIdx.x * a.t.nsamples + n] = h.v[threadIdx.x];
+    __syncthreads();  // the samples are stored, and every thread has read the step
+    if (n < a.t.nsamples)
+        for (int u = threadIdx.x; u < a.t.ngroup; u += blockDim.x) add_source_group(a.t, u, n, a.cur);
+    if (threadIdx.x == 0) {
+        a.ctr[1] = n;
+        a.ctr[0] = n + a.advance;
+    }
+}
+
+// A few receiver rows straight into pinned host memory: latency only.
+__global__ void k_rows_out(const float *rows, float *out, int n)
+{
+    grid_dependency_wait();
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = rows[i];
+}
+
+__global__ void k_zero(const ZeroArgs z)
+{
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+    {
+        float4 *v = reinterpret_cast<float4 *>(z.f[k]);
+        const int64_t n4 = z.n[k] >> 2;
+        for (int64_t i = t; i < n4; i += step) v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        const int64_t i = 4 * n4 + t;
+        if (i < z.n[k]) z.f[k][i] = 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < 2; k++)
+        if (t < z.ni[k]) z.i[k][t] = 0;
+}
+
 // REF: the reference's update arithmetic, (2 p^n - p^{n-1}) - ((dt*dt) y) / M, each operation
 // rounded (SEMsolver.cpp:85-89), with M in a.mref; otherwise the precomputed a = dt^2/M.
 template <bool SPONGE, bool REF>
@@ -316,6 +357,26 @@ cudaError_t launch_mass_ref(float *m, const float *vel, int ex, int ey, int ez, 
 cudaError_t launch_source(const SourceArgs &a, cudaStream_t s, bool after)
 {
     return launch_after(k_source, dim3(1), a.t.ngroup > 32 ? 256 : 32, 0, s, after, a);
+}
+
+cudaError_t launch_source_samples(const SourceArgs &a, const HostSamples &h, float *wavelet, cudaStream_t s)
+{
+    if (h.n < 0 || h.n > kMaxHostSamples) return cudaErrorInvalidValue;
+    k_source_samples<<<1, 32, 0, s>>>(a, h, wavelet);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_rows_out(const float *rows, float *out, int n, cudaStream_t s, bool dependent)
+{
+    return launch_after(k_rows_out, dim3((unsigned)std::min((n + 255) / 256, 152)), 256, 0, s, dependent, rows, out, n);
+}
+
+cudaError_t launch_zero(const ZeroArgs &z, cudaStream_t s)
+{
+    int64_t n = 1;
+    for (int k = 0; k < 4; k++) n = std::max(n, z.n[k]);
+    k_zero<<<(unsigned)std::min<int64_t>((n + 1023) / 1024, 152 * 8), 256, 0, s>>>(z);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_connectivity(int32_t *conn, int ex, int ey, int ez, int order, int64_t nxp,

@@ -83,6 +83,14 @@ struct SourceArgs {
     int advance;  // steps until the next source launch (the passes between add their own sources)
 };
 
+// One step's samples of all sources, handed to the source launch by value (sem_solver_step_host): the
+// launch stores them in the wavelets' column of the step and adds them.  32: one thread each in one warp.
+constexpr int kMaxHostSamples = 32;
+struct HostSamples {
+    int n;
+    float v[kMaxHostSamples];
+};
+
 #ifdef __CUDACC__
 // The sources of step n on one node (group u of the table).
 __device__ __forceinline__ void add_source_group(const SourceTable &t, int u, int n, float *level)
@@ -107,6 +115,18 @@ cudaError_t launch_element(int order, const ElementArgs &a, cudaStream_t s);  //
 cudaError_t launch_update(const UpdateArgs &a, bool sponge, cudaStream_t s);
 // after: as a programmatic dependent of the preceding kernel of the stream
 cudaError_t launch_source(const SourceArgs &a, cudaStream_t s, bool after = false);
+// As launch_source, with the step's samples of the sources written to `wavelet` (a.t.wavelet) first.
+cudaError_t launch_source_samples(const SourceArgs &a, const HostSamples &h, float *wavelet, cudaStream_t s);
+// out[0..n) = rows[0..n) (out: pinned host memory as the device sees it); dependent: see launch.cuh.
+cudaError_t launch_rows_out(const float *rows, float *out, int n, cudaStream_t s, bool dependent);
+// Zeroes up to four arrays of floats (16-byte aligned; n 0: none) and two of ints in one launch.
+struct ZeroArgs {
+    float *f[4];
+    int64_t n[4];
+    int *i[2];
+    int ni[2];
+};
+cudaError_t launch_zero(const ZeroArgs &z, cudaStream_t s);
 cudaError_t launch_connectivity(int32_t *conn, int ex, int ey, int ez, int order, int64_t nxp,
                                 cudaStream_t s);
 // Gradient with respect to the nodal mass parameter -> with respect to squared slowness: g /= m.

@@ -41,6 +41,7 @@ struct sem_solver {
     // sponge
     bool sponge = false;
     float *d_sx = nullptr, *d_sy = nullptr, *d_sz = nullptr;
+    float *pin = nullptr, *d_pin = nullptr;  // pinned staging of receiver rows (sem_solver_step_host)
     // sources
     int nsrc = 0, nsamples = 0;
     int64_t *d_src_node = nullptr;
@@ -80,6 +81,7 @@ struct StepExtra {
     // preceding kernel on the stream belongs to the run
     int advance = 1, step_off = 0;
     bool inject = false, after = false;
+    const semgb::HostSamples *samples = nullptr;  // this step's source samples, by value (advance 1)
 };
 
 // Device resources for stepping n_new more steps (mass, stencil tables, receiver CSR, trace

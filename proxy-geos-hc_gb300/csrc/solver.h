@@ -41,6 +41,7 @@ struct sem_solver {
     // sponge
     bool sponge = false;
     float *d_sx = nullptr, *d_sy = nullptr, *d_sz = nullptr;
+    std::vector<float> h_sx, h_sy, h_sz;  // the same on the host
     float *pin = nullptr, *d_pin = nullptr;  // pinned staging of receiver rows (sem_solver_step_host)
     // sources
     int nsrc = 0, nsamples = 0;

@@ -101,7 +101,7 @@ struct RowSmem {
     alignas(16) float z2[NROW * HS];
     float d[NROW];
     // boundary: features (then inputs), feature gradient, per-row scale, arg-max, node coordinates
-    alignas(16) float xf[BOUNDARY ? NROW * KX4 : 4];
+    alignas(16) float xf[BOUNDARY ? NROW * (KX4 + 1) : 4];
     alignas(16) float dx[BOUNDARY ? NROW * (KX4 + 1) : 4];
     float scale[BOUNDARY ? NROW : 1], gb[BOUNDARY ? NROW : 1], y[BOUNDARY ? NROW : 1];
     int kstar[BOUNDARY ? NROW : 1];
@@ -283,6 +283,10 @@ __global__ void __launch_bounds__(8 * NROW) k_mlp_rows(const MlpDev net, const S
 // the 81 features of the node from the recorded levels, divided by their largest magnitude; the
 // forward; dy = g scale where the output is not clipped; the backward down to the inputs; and
 // the feature gradient G = dx / scale plus the scale's share on its arg-max feature.
+// A box of 12^3 elements of order 4 is one wave of 32-row CTAs, so what counts is a CTA's chain of phases:
+// the node coordinates before the wait, a row's features by eight threads with all loads in flight and
+// kept in registers to the inputs, dx in packed f32x2 (scalar: 21.5 us) and scaled where it is formed.
+// 24.3 -> 20.1 us a launch; with a pass per phase through shared memory the features took 7 k of the 36 k cycles.
 template <int NROW>
 __global__ void __launch_bounds__(8 * NROW, 3) k_mlp_boundary(const MlpDev net, const BpttFields f, const float *lm,
                                                            const float *lm1, const float *lm2, const MlpWork wk,
@@ -292,72 +296,86 @@ __global__ void __launch_bounds__(8 * NROW, 3) k_mlp_boundary(const MlpDev net, 
     RowSmem<NROW, true> &s = *reinterpret_cast<RowSmem<NROW, true> *>(smem);
     const int tid = threadIdx.x;
     copy_net(s.net, net);  // constant over the time loop: staged before the wait
+    const int64_t plane = f.nxp * f.nz;
+    // coordinates of a tile's nodes (the node list is constant too)
+    auto place = [&](int64_t rg) {
+        if (tid >= NROW) return;
+        const int64_t b = row0 + rg + tid;
+        int4 c = make_int4(0, 0, 0, 0);
+        if (b < f.nb) {
+            const int64_t q = f.nodes[b];
+            const int iy = (int)(q / plane);
+            const int64_t r = q - (int64_t)iy * plane;
+            const int iz = (int)(r / f.nxp);
+            c = make_int4((int)(r - (int64_t)iz * f.nxp), iy, iz, 1);
+        }
+        s.at[tid] = c;
+    };
+    int64_t rg = (int64_t)blockIdx.x * NROW;
+    if (rg < rows) place(rg);
     copies_landed();
     grid_dependency_wait();
-    const int64_t plane = f.nxp * f.nz;
-    for (int64_t rg = (int64_t)blockIdx.x * NROW; rg < rows; rg += (int64_t)gridDim.x * NROW) {
-        __syncthreads();  // the previous rows are stored
-        if (tid < NROW) {
-            const int64_t b = row0 + rg + tid;
-            int4 c = make_int4(0, 0, 0, 0);
-            if (b < f.nb) {
-                const int64_t q = f.nodes[b];
-                const int iy = (int)(q / plane);
-                const int64_t r = q - (int64_t)iy * plane;
-                const int iz = (int)(r / f.nxp);
-                c = make_int4((int)(r - (int64_t)iz * f.nxp), iy, iz, 1);
-                s.gb[tid] = f.a[0][q];
-            }
-            s.at[tid] = c;
+    for (; rg < rows; rg += (int64_t)gridDim.x * NROW) {
+        if (rg >= (int64_t)gridDim.x * NROW) {
+            __syncthreads();  // the previous rows are stored
+            place(rg);
         }
         __syncthreads();
-        // features: level 0 (what the step leaves before the network: s (s q) on the boundary), 1, 2
-        for (int i = tid; i < NROW * 27; i += 8 * NROW) {
-            const int r = i / 27, nbh = i - r * 27;
-            const int4 c = s.at[r];
-            const int jx = c.x + nbh % 3 - 1, jy = c.y + (nbh / 3) % 3 - 1, jz = c.z + nbh / 9 - 1;
-            float f0 = 0.f, f1 = 0.f, f2 = 0.f;
-            if (c.w && jx >= 0 && jx < f.nx && jy >= 0 && jy < f.ny && jz >= 0 && jz < f.nz) {
-                const int64_t qn = jx + (int64_t)jz * f.nxp + (int64_t)jy * plane;
-                const float sj = f.sx ? (f.sx[jx] * f.sz[jz]) * f.sy[jy] : 1.f;
-                const bool bnd = jx == 0 || jx == f.nx - 1 || jy == 0 || jy == f.ny - 1 || jz == 0 || jz == f.nz - 1;
-                const float hq = lm2[qn] * sj;  // s q: the history the step keeps
-                f0 = bnd ? hq * sj : lm[qn];
-                f1 = lm1[qn] * sj;
-                f2 = hq;
-            }
-            float *xr = s.xf + r * KX4;
-            xr[nbh] = f0;
-            xr[27 + nbh] = f1;
-            xr[54 + nbh] = f2;
-        }
-        __syncthreads();
-        // largest magnitude and its first feature, eight threads per row; then the inputs
+        // Features, eight threads per row, four neighbours of three levels each with all their loads in
+        // flight: level 0 (what the step leaves before the network: s (s q) on the boundary), 1, 2.
+        // Their largest magnitude and its first feature over the eight threads, then the inputs.
         {
             const int r = tid >> 3, p = tid & 7;
+            const int4 c = s.at[r];
+            float v[3][4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const int nbh = p + 8 * j;
+                const int jx = c.x + nbh % 3 - 1, jy = c.y + (nbh / 3) % 3 - 1, jz = c.z + nbh / 9 - 1;
+                v[0][j] = v[1][j] = v[2][j] = 0.f;
+                if (c.w && nbh < 27 && jx >= 0 && jx < f.nx && jy >= 0 && jy < f.ny && jz >= 0 && jz < f.nz) {
+                    const int64_t qn = jx + (int64_t)jz * f.nxp + (int64_t)jy * plane;
+                    const float sj = f.sx ? (f.sx[jx] * f.sz[jz]) * f.sy[jy] : 1.f;
+                    const bool bnd = jx == 0 || jx == f.nx - 1 || jy == 0 || jy == f.ny - 1 || jz == 0 || jz == f.nz - 1;
+                    const float q0 = lm[qn], q1 = lm1[qn], q2 = lm2[qn];
+                    const float hq = q2 * sj;  // s q: the history the step keeps
+                    v[0][j] = bnd ? hq * sj : q0;
+                    v[1][j] = q1 * sj;
+                    v[2][j] = hq;
+                }
+            }
+            if (p == 7 && c.w) s.gb[r] = f.a[0][c.x + (int64_t)c.z * f.nxp + (int64_t)c.y * plane];
             float m = 0.f;
-            int km = 0;
-            float *xr = s.xf + r * KX4;
-            for (int k = p; k < kMlpIn; k += 8)
-                if (fabsf(xr[k]) > m) { m = fabsf(xr[k]); km = k; }
+            int km = 0;  // the feature, 0x100: negative
+#pragma unroll
+            for (int l = 0; l < 3; l++)
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    if (fabsf(v[l][j]) > m) { m = fabsf(v[l][j]); km = (27 * l + p + 8 * j) | (v[l][j] < 0.f ? 0x100 : 0); }
 #pragma unroll
             for (int o = 1; o < 8; o <<= 1) {
                 const float mo = __shfl_xor_sync(0xffffffffu, m, o);
                 const int ko = __shfl_xor_sync(0xffffffffu, km, o);
-                if (mo > m || (mo == m && ko < km)) { m = mo; km = ko; }
+                if (mo > m || (mo == m && (ko & 0xff) < (km & 0xff))) { m = mo; km = ko; }
             }
             const float sc = m + 1e-30f, inv = 1.f / sc;
             if (p == 0) {
                 s.scale[r] = sc;
                 // -1: an all-zero neighbourhood (the value is 0 there, its gradient taken as 0)
-                s.kstar[r] = m > 0.f ? (km | (xr[km] < 0.f ? 0x100 : 0)) : -1;
+                s.kstar[r] = m > 0.f ? km : -1;
             }
-            __syncwarp();
-            for (int k = p; k < kMlpInPad; k += 8) {
-                const float v = k < kMlpIn ? xr[k] * inv : 0.f;
-                if (k < kMlpIn) xr[k] = v;
-                s.xs[r * KP1 + k] = f2bf(v);
-            }
+#pragma unroll
+            for (int l = 0; l < 3; l++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const int k = 27 * l + p + 8 * j;
+                    if (p + 8 * j < 27) {
+                        const float x = v[l][j] * inv;
+                        s.xf[r * DXS + k] = x;
+                        s.xs[r * KP1 + k] = f2bf(x);
+                    }
+                }
+            for (int k = kMlpIn + p; k < kMlpInPad; k += 8) s.xs[r * KP1 + k] = 0;
         }
         __syncthreads();
         rows_backward<NROW, true>(s, wk.g2 + rg * H, [&](int r, float y) {
@@ -366,14 +384,16 @@ __global__ void __launch_bounds__(8 * NROW, 3) k_mlp_boundary(const MlpDev net, 
             return (y > -1.f && y < 1.f) ? s.gb[r] * s.scale[r] : 0.f;
         });
         store_rows<NROW, true>(s, wk, rg);
-        // dx[k] = sum_n dZ1[n] W1[n][k]: four rows and four inputs per thread
+        // dx[k] = sum_n dZ1[n] W1[n][k], divided by the scale: four rows and four inputs per thread
         if (tid < NROW / 4 * (KX4 / 4)) {
             const int r = tid / (KX4 / 4) * 4, k = tid % (KX4 / 4) * 4;
-            float d[4][4];
+            float d[4][4], inv[4];
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < 4; i++) {
+                inv[i] = 1.f / s.scale[r + i];
 #pragma unroll
                 for (int j = 0; j < 4; j++) d[i][j] = 0.f;
+            }
 #pragma unroll 2
             for (int n = 0; n < H; n += 4) {
                 float a[4][4];
@@ -387,32 +407,30 @@ __global__ void __launch_bounds__(8 * NROW, 3) k_mlp_boundary(const MlpDev net, 
                     const float4 w4 = bf4(s.net.w1 + (n + j) * KP1 + k);
 #pragma unroll
                     for (int i = 0; i < 4; i++) {
-                        d[i][0] = fmaf(a[i][j], w4.x, d[i][0]); d[i][1] = fmaf(a[i][j], w4.y, d[i][1]);
-                        d[i][2] = fmaf(a[i][j], w4.z, d[i][2]); d[i][3] = fmaf(a[i][j], w4.w, d[i][3]);
+                        const float2 aa = make_float2(a[i][j], a[i][j]);
+                        const float2 u = fma2(aa, make_float2(w4.x, w4.y), make_float2(d[i][0], d[i][1]));
+                        const float2 v = fma2(aa, make_float2(w4.z, w4.w), make_float2(d[i][2], d[i][3]));
+                        d[i][0] = u.x; d[i][1] = u.y; d[i][2] = v.x; d[i][3] = v.y;
                     }
                 }
             }
 #pragma unroll
             for (int i = 0; i < 4; i++)
 #pragma unroll
-                for (int j = 0; j < 4; j++) s.dx[(r + i) * DXS + k + j] = d[i][j];
+                for (int j = 0; j < 4; j++) s.dx[(r + i) * DXS + k + j] = d[i][j] * inv[i];
         }
         __syncthreads();
-        // feature gradient in place of dx: the division by the scale, and the scale's own share
+        // the scale's own share of the feature gradient: one thread per row, features in order
         if (tid < NROW && row0 + rg + tid < f.nb) {
-            const float *xr = s.xf + tid * KX4;
+            const float *xr = s.xf + tid * DXS;
             float *d = s.dx + tid * DXS;
             const int ks = s.kstar[tid];
             if (ks < 0) {
                 for (int k = 0; k < kMlpIn; k++) d[k] = 0.f;
             } else {
-                const float inv = 1.f / s.scale[tid];
                 float xd = 0.f;
-#pragma unroll 9
-                for (int k = 0; k < kMlpIn; k++) {
-                    d[k] *= inv;
-                    xd = fmaf(xr[k], d[k], xd);
-                }
+#pragma unroll 27
+                for (int k = 0; k < kMlpIn; k++) xd = fmaf(xr[k], d[k], xd);
                 const float h = fminf(fmaxf(s.y[tid], -1.f), 1.f);
                 const float sg = (ks & 0x100) ? -1.f : 1.f;
                 d[ks & 0xff] += sg * (s.gb[tid] * h - xd);

@@ -84,7 +84,8 @@ struct Cfg {
     static constexpr int AUX_FLOATS = 2 * TILE_FLOATS + WIN_FLOATS;  // p^{n-1}, dt^2/M tiles; p^n window
     static constexpr size_t OFF_AUX = (size_t)R * RING_FLOATS * 4;
     static constexpr size_t OFF_BAR = OFF_AUX + (size_t)AUX * AUX_FLOATS * 4;
-    static constexpr size_t SMEM = OFF_BAR + 8 * (R + AUX);
+    static constexpr size_t OFF_OWN = OFF_BAR + 8 * (R + AUX);  // order 1: see `own` of the CTA
+    static constexpr size_t SMEM = OFF_OWN + (O == 1 ? 8 : 0);
     static constexpr uint32_t RING_TX = sizeof(float) * TZ * TX;
     static constexpr uint32_t AUX_TX = sizeof(float) * (2 * TZ * TX + TZP * TXP);
     // CTAs per SM that shared memory allows (228 KB per SM, 1 KB reserved per CTA), at most 6;
@@ -401,6 +402,12 @@ __device__ __forceinline__ void stencil_cta(const CUtensorMap *rmap, const CUten
     float *ring = reinterpret_cast<float *>(smem);
     float *aux = reinterpret_cast<float *>(smem + C::OFF_AUX);
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + C::OFF_BAR);  // [R] ring, [AUX] aux
+    // Whether the CTA's nodes hold sources and receivers.  Order 1 looks it up while the first planes load: its
+    // CTAs are short (801^3 nodes: 31 waves), and the dependent loads at the end of the march kept each
+    // one's slot: 1459 us a step, 1425 so; 301^3 88.3, 84.4; 101^3 7.2, 6.9.  The longer CTAs of the other orders lost
+    // more at the start (order 2: 40^3 elements 4.7 us, 5.1 so; order 4: 61x70x53 48.9, 49.5).
+    constexpr bool EARLY = O == 1 && !MULTI && !GROUP;
+    int *own = reinterpret_cast<int *>(smem + C::OFF_OWN);
 
     const bool act = !GROUP || threadIdx.x < (unsigned)C::THREADS;  // a thread of the configuration
     const int tid = act ? (int)threadIdx.x : 0;  // extra threads shadow thread 0 and store nothing
@@ -429,6 +436,7 @@ __device__ __forceinline__ void stencil_cta(const CUtensorMap *rmap, const CUten
     if (threadIdx.x == 0) {
         for (int i = 0; i < R + AUX; i++) bar_init(bars + i, 1);
         fence_barrier_init();
+        if constexpr (EARLY) own[0] = own[1] = 0;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -484,6 +492,13 @@ __device__ __forceinline__ void stencil_cta(const CUtensorMap *rmap, const CUten
                            t.grid[0], t.grid[1],
                            t.far_x, t.far_z},
                   bx, bz, yb, ye - yb);
+    if constexpr (EARLY) {
+        // from the last thread down: thread 0 has just issued the copies
+        const int c = bx + t.grid[0] * (bz + t.grid[1] * chunk), rev = C::THREADS - 1 - (int)threadIdx.x;
+        for (int u = rev; inject && u < a.src.ngroup; u += C::THREADS)
+            if (a.src_cta[u] == c) own[0] = 1;
+        if (a.nrec > 0 && rev == 1 && a.rec_off[c] < a.rec_off[c + 1]) own[1] = 1;
+    }
     bool ok = true;
     for (int p = yb - O; p < yb + O; p++) {
         const int i = p - yb + O;  // < 2O < R: first fill of each of these slots
@@ -721,7 +736,7 @@ __device__ __forceinline__ void stencil_cta(const CUtensorMap *rmap, const CUten
         return;
     }
     const int cta = bx + t.grid[0] * (bz + t.grid[1] * chunk);  // tile and chunk
-    if (a.nrec > 0) {
+    if (EARLY ? own[1] != 0 : a.nrec > 0) {
         const int r0 = a.rec_off[cta], r1 = a.rec_off[cta + 1];
         if (r0 < r1) {  // uniform over the CTA; its new values are visible after the last barrier
             const int step = a.ctr[1] + step_off;
@@ -734,7 +749,7 @@ __device__ __forceinline__ void stencil_cta(const CUtensorMap *rmap, const CUten
             }
         }
     }
-    if (inject && a.src.ngroup > 0) {
+    if (EARLY ? own[0] != 0 : inject && a.src.ngroup > 0) {
         const int n = a.ctr[1] + step_off + 1;
         __syncthreads();  // the receivers above have sampled the level without the next sources
         if (n < a.src.nsamples) {

@@ -384,9 +384,8 @@ int sem_adjoint_get_adjoint_traces(sem_adjoint *a, float *out);
 /* One element-path step (K.p by the element kernel, then the leapfrog update) on buffers the
  * caller owns, for callers that cannot allocate device memory while they step -- a host code
  * that gives all device memory to its own pool manager, or one whose time loop runs where
- * allocation is not allowed.  The call allocates nothing: the K.p accumulator and a small
- * coefficient table live in a fixed array of 4,194,304 floats (16 MiB) in the library's device
- * image, so the mesh may have at most 4,194,176 nodes; larger meshes are rejected with
+ * allocation is not allowed.  The call allocates nothing: the K.p accumulator lives in a fixed
+ * array of 4,194,304 floats (16 MiB) in the library's device image, so the mesh may have at most 4,194,176 nodes; larger meshes are rejected with
  * SEM_ERR_ARG.  All buffers are device memory in the reference node numbering:
  *   conn    int32 [n_elem][(order+1)^3] element-to-node map (as sem_mesh_get_connectivity gives);
  *           entries must lie in [0, n_nodes): one outside is skipped (read as 0, not scattered)
@@ -402,8 +401,8 @@ int sem_adjoint_get_adjoint_traces(sem_adjoint *a, float *out);
  * before the caller's pool manager reserves device memory, and before any stream capture; later
  * calls leave the device's free memory unchanged.  The cached address does not survive
  * cudaDeviceReset (nor does any other handle of this library).  Every call uses the same array,
- * which keeps the last call's contents (the call clears what it needs): calls whose work
- * overlaps on the GPU race on it. */
+ * which is zero between calls (the update clears behind itself; after a call that failed to
+ * launch the next one clears it first): calls whose work overlaps on the GPU race on it. */
 int sem_element_step_noalloc(int ex, int ey, int ez, float lx, float ly, float lz, int order,
                              const int32_t *conn, float *p_cur, float *p_prev, const float *coef,
                              const float *sx, const float *sy, const float *sz, void *stream);
@@ -469,7 +468,8 @@ int sem_abc_features(sem_abc *a, float *x, float *scale);
  * Sources must lie at least two nodes inside the box.  The solver is left after the n_steps.
  * Every level is recorded: (n_steps + 2) x (the mesh's device-layout node count) floats of
  * device memory, plus a few fields, for the duration of the call (meant for training regions;
- * SEM_ERR_OOM when it does not fit). */
+ * SEM_ERR_OOM when it does not fit); the network's work arrays (at most 86 MB) stay with the
+ * network. */
 int sem_abc_bptt(sem_abc *a, int n_steps, int n_roi, const int64_t *roi_nodes, const float *ref, double *loss,
                  float *grad);
 

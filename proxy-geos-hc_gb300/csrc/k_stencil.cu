@@ -6,7 +6,9 @@
 // along the same axis (zero outside the node's element or element pair), applied in difference
 // form sum_d T[l][d] (p_{i+d} - p_i), exactly zero for a constant field.
 //
-// Work decomposition (HBM-bound pass: read p^n, p^{n-1}, dt^2/M, write p^{n+1}; 16 B/node):
+// Work decomposition (16 B/node: read p^n, p^{n-1}, dt^2/M, write p^{n+1}; 89 % of the copy rate at 200^3
+// elements of order 4, there and below bound by the latency of a plane -- one barrier, its shared-memory
+// loads -- at 12 warps per SM: cutting DRAM traffic or shared-memory loads alone changed nothing):
 //  - a CTA owns a tile of TX nodes along x by TZ rows along z and marches along y over a chunk
 //    of planes; a lane holds one element's o consecutive x-nodes, so a node's local x index is a
 //    compile-time constant (x-coefficients are immediates, zero terms are skipped); a warp covers

@@ -35,6 +35,11 @@ struct sem_batch {
     int64_t *d_src_node = nullptr;
     float *d_src_coef = nullptr;
     float *d_wavelet = nullptr;
+    // a batch of one shot runs the single-shot pass, whose sources are grouped by node and looked up by
+    // owning CTA (SourceTable); many shots need neither and leave these empty
+    int *d_src_off = nullptr, *d_src_perm = nullptr;
+    std::vector<int64_t> src_group;
+    uint64_t src_version = 1;
     int nrec = 0;
     std::vector<int64_t> rec_sorted;  // device-layout nodes, sorted
     int64_t *d_rec_node = nullptr;
@@ -81,25 +86,28 @@ StencilArgs args_for(const sem_batch *b, int c, bool record)
 cudaError_t enqueue(sem_batch *b, int c, int n)
 {
     const int nsrc = b->nsamples > 0 ? b->nshot : 0;
+    const int ngroup = b->nsamples <= 0 ? 0 : b->nshot > 1 ? b->nshot : (int)b->src_group.size();
     cudaError_t e = launch_batch_source(BatchSourceArgs{b->d_p[c], b->d_src_node, b->d_src_coef, b->d_wavelet, nsrc,
                                                         b->nsamples, b->n_int, b->d_ctr, n}, b->stream);
     for (int k = 0; k < n && e == cudaSuccess; k++, c ^= 1) {
         StencilArgs a = args_for(b, c, true);
         a.step_off = k;
         a.inject = k + 1 < n;
-        a.src = SourceTable{b->d_src_node, b->d_src_coef, b->d_wavelet, nullptr, nullptr, nsrc, b->nsamples};
+        a.src = SourceTable{b->d_src_node, b->d_src_coef, b->d_wavelet, b->d_src_off, b->d_src_perm, ngroup, b->nsamples};
+        a.src_cta = b->st->d_src_cta;
         e = launch_stencil(*b->st, a, c, b->sponge, b->stream, STENCIL_PLAIN, true, true);
     }
     return e;
 }
 
-// Sets the stencil pass's y-chunk (planes per CTA) and regroups the receivers by CTA.
+// Sets the stencil pass's y-chunk (planes per CTA) and regroups the receivers and sources by CTA.
 cudaError_t set_chunk(sem_batch *b, int ychunk)
 {
     StencilTables &t = *b->st;
     t.ychunk = std::max(1, std::min<int>(ychunk, (int)t.ny));
     t.grid[2] = (int)((t.ny + t.ychunk - 1) / t.ychunk);
-    return stencil_set_receivers(t, b->rec_sorted.data(), b->nrec, b->rec_version);
+    cudaError_t e = stencil_set_receivers(t, b->rec_sorted.data(), b->nrec, b->rec_version);
+    return e == cudaSuccess ? stencil_set_sources(t, b->src_group, b->src_version) : e;
 }
 
 int prepare(sem_batch *b, int64_t n_new)
@@ -114,6 +122,10 @@ int prepare(sem_batch *b, int64_t n_new)
         return sem_fail(SEM_ERR_CUDA, "tensor-map encoding failed (driver entry point cuTensorMapEncodeTiled)");
     if (b->st->rec_version != b->rec_version) {
         CUDA_TRY(stencil_set_receivers(*b->st, b->rec_sorted.data(), b->nrec, b->rec_version));
+        invalidate(b);
+    }
+    if (b->st->src_version != b->src_version) {
+        CUDA_TRY(stencil_set_sources(*b->st, b->src_group, b->src_version));
         invalidate(b);
     }
     if (b->nrec > 0 && b->steps_done + n_new > b->trace_cap) {
@@ -160,6 +172,7 @@ int sem_batch_destroy(sem_batch *b)
     dfree(b->d_w);
     dfree(b->d_sx); dfree(b->d_sy); dfree(b->d_sz);
     dfree(b->d_src_node); dfree(b->d_src_coef); dfree(b->d_wavelet);
+    dfree(b->d_src_off); dfree(b->d_src_perm);
     dfree(b->d_rec_node);
     dfree(b->d_rec_perm);
     dfree(b->d_traces);
@@ -279,15 +292,27 @@ int sem_batch_set_sources(sem_batch *b, const int64_t *elements, const float *wa
     cudaStreamSynchronize(b->stream);
     invalidate(b);
     dfree(b->d_src_node); dfree(b->d_src_coef); dfree(b->d_wavelet);
+    dfree(b->d_src_off); dfree(b->d_src_perm);
+    b->nsamples = 0;  // until the arrays are in place
+    b->src_group.clear();
+    b->src_version++;
+    if (b->nshot == 1 && node[0] >= 0) {
+        const int off[2] = {0, 1}, perm[1] = {0};
+        CUDA_TRY(dalloc(&b->d_src_off, 2));
+        CUDA_TRY(dalloc(&b->d_src_perm, 1));
+        CUDA_TRY(cudaMemcpy(b->d_src_off, off, sizeof(off), cudaMemcpyHostToDevice));
+        CUDA_TRY(cudaMemcpy(b->d_src_perm, perm, sizeof(perm), cudaMemcpyHostToDevice));
+        b->src_group.push_back(node[0]);
+    }
     CUDA_TRY(dalloc(&b->d_src_node, b->nshot));
     CUDA_TRY(dalloc(&b->d_src_coef, b->nshot));
     CUDA_TRY(cudaMemcpy(b->d_src_node, node.data(), b->nshot * 8, cudaMemcpyHostToDevice));
     CUDA_TRY(cudaMemcpy(b->d_src_coef, coef.data(), b->nshot * 4, cudaMemcpyHostToDevice));
-    b->nsamples = n_samples;
     if (n_samples > 0) {
         CUDA_TRY(dalloc(&b->d_wavelet, (size_t)b->nshot * n_samples));
         CUDA_TRY(cudaMemcpy(b->d_wavelet, wavelet, (size_t)b->nshot * n_samples * 4, cudaMemcpyHostToDevice));
     }
+    b->nsamples = n_samples;
     return SEM_OK;
     GUARD_END
 }

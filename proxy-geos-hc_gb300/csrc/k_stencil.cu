@@ -445,6 +445,10 @@ cudaError_t launch_stencil(const StencilTables &t, const StencilArgs &a, int cur
                            int mode, bool direct, bool after)
 {
     if (mode != STENCIL_PLAIN && (!a.kp || (mode == STENCIL_GRADIENT && !a.grad))) return cudaErrorInvalidValue;
+    // a pass that adds the next step's sources reads their table on the device: the single-shot one all of it
+    if (a.inject && a.src.ngroup > 0 &&
+        (!a.src.node || !a.src.coef || !a.src.wavelet || (t.nshot <= 1 && (!a.src.off || !a.src.perm || !a.src_cta))))
+        return cudaErrorInvalidValue;
     switch (t.order) {
     case 1: return launch_o<1>(t, a, cur_index, sponge, mode, direct, s, after);
     case 2: return launch_o<2>(t, a, cur_index, sponge, mode, direct, s, after);

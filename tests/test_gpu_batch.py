@@ -69,3 +69,43 @@ def test_batch_autotune_keeps_state(semgb_lib, cuda_device):
         b.close()
     assert np.array_equal(res[1][0], res[0][0])
     assert np.array_equal(res[1][1], res[0][1])
+
+
+@pytest.mark.parametrize("order", [1, 2, 3, 4, 5])
+def test_batch_of_one_shot_matches_plain_solver(semgb_lib, cuda_device, order):
+    """One shot is the plain pass with the batch's own tables: runs of 1, 2, 16 and 17 steps, with a source,
+    with a wavelet but no source, and with no wavelet; and again after the autotuner has changed the
+    chunks (and with them the CTA that owns the source)."""
+    semgb = semgb_lib
+    wl, wav = _setup(semgb, order, 1, seed=80 + order)
+    element = semgb.element_from_point(wl.ex, wl.ey, wl.ez, wl.lx, wl.ly, wl.lz, *wl.src_xyz[0])
+    mesh = semgb.Mesh(wl.ex, wl.ey, wl.ez, wl.lx, wl.ly, wl.lz, order)
+    mesh.set_velocity(wl.vel)
+    for kind in ("source", "none", "no wavelet"):
+        b = semgb.Batch(mesh, wl.dt, 1)
+        p = semgb.Solver(mesh, wl.dt)
+        p.set_kernel(semgb.KERNEL_STENCIL)
+        p.set_tile_shape(semgb.TILE_DEFAULT)
+        for s in (b, p):
+            s.set_sponge(wl.sponge_thickness, wl.sponge_sigma)
+            s.set_receivers(wl.rec_xyz)
+        if kind == "source":
+            b.set_sources([element], wav)
+            p.set_sources([element], wav)
+        elif kind == "none":
+            b.set_sources([-1], wav)
+        done = 0
+        for k, n in enumerate((1, 2, 16, 17)):
+            if k == 3:
+                b.autotune()
+            b.step(n)
+            p.step(n)
+            done += n
+            b.synchronize()
+            got, want = b.traces(), p.traces()
+            assert got.shape == (done, 9, 1) and np.array_equal(got[:, :, 0], want), (kind, n)
+            assert np.array_equal(b.pressure(0), p.pressure()), (kind, n)
+            assert np.array_equal(b.pressure(0, semgb.LEVEL_PREVIOUS), p.pressure(semgb.LEVEL_PREVIOUS)), (kind, n)
+        assert (np.abs(b.pressure(0)).max() > 0) == (kind == "source")
+        b.close()
+        p.close()

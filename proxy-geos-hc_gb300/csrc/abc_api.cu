@@ -282,7 +282,7 @@ int sem_mlp_forward(sem_mlp *m, int64_t n, const float *x, float *y)
     float *dx = nullptr, *dy = nullptr;
     CUDA_TRY(dalloc(&dx, (size_t)n * kMlpIn));
     cudaError_t e = dalloc(&dy, (size_t)n);
-    if (e == cudaSuccess) e = cudaMemcpy(dx, x, (size_t)n * kMlpIn * 4, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = upload(dx, x, (size_t)n * kMlpIn, m->stream);
     if (e == cudaSuccess) e = mlp_forward(m->dev(), dx, dy, n, m->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
     if (e == cudaSuccess) e = cudaMemcpy(y, dy, (size_t)n * 4, cudaMemcpyDeviceToHost);
@@ -300,8 +300,8 @@ int sem_mlp_loss_grad(sem_mlp *m, int64_t n, const float *x, const float *t, dou
     float *dx = nullptr, *dt = nullptr;
     CUDA_TRY(dalloc(&dx, (size_t)n * kMlpIn));
     cudaError_t e = dalloc(&dt, (size_t)n);
-    if (e == cudaSuccess) e = cudaMemcpy(dx, x, (size_t)n * kMlpIn * 4, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(dt, t, (size_t)n * 4, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = upload(dx, x, (size_t)n * kMlpIn, m->stream);
+    if (e == cudaSuccess) e = upload(dt, t, n, m->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(m->d_grad, 0, kMlpParams * 4, m->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(m->d_loss, 0, 8, m->stream);
     if (e == cudaSuccess) e = ensure_work(m, n);
@@ -437,9 +437,9 @@ int sem_abc_create(sem_solver *s, sem_mlp *net, int layer_elems, sem_abc **out)
     if (e == cudaSuccess) e = dalloc(&a->d_shell, shell.size());
     if (e == cudaSuccess) e = dalloc(&a->d_hist, (size_t)b.n_int);
     if (e == cudaSuccess) e = dalloc(&a->d_corr, nodes.size());
-    if (e == cudaSuccess) e = cudaMemcpy(a->d_nodes, nodes.data(), nodes.size() * 8, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(a->d_shell, shell.data(), shell.size() * 8, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(a->d_hist, 0, (size_t)b.n_int * 4);
+    if (e == cudaSuccess) e = upload(a->d_nodes, nodes.data(), nodes.size(), s->stream);
+    if (e == cudaSuccess) e = upload(a->d_shell, shell.data(), shell.size(), s->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(a->d_hist, 0, (size_t)b.n_int * 4, s->stream);
     if (e == cudaSuccess && layer_elems == 0) {
         // face tiles: y-faces whole, z-faces without the rows on y-faces, x-faces without the
         // rows on y- and z-faces, so every boundary node lies on one face
@@ -464,8 +464,8 @@ int sem_abc_create(sem_solver *s, sem_mlp *net, int layer_elems, sem_abc **out)
         a->ntiles = (int64_t)tiles.size();
         e = dalloc(&a->d_tiles, tiles.size());
         if (e == cudaSuccess) e = dalloc(&a->d_hist_alt, (size_t)b.n_int);
-        if (e == cudaSuccess) e = cudaMemcpy(a->d_tiles, tiles.data(), tiles.size() * sizeof(int4), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemset(a->d_hist_alt, 0, (size_t)b.n_int * 4);
+        if (e == cudaSuccess) e = upload(a->d_tiles, tiles.data(), tiles.size(), s->stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(a->d_hist_alt, 0, (size_t)b.n_int * 4, s->stream);
     }
     if (e != cudaSuccess) {
         sem_abc_destroy(a);
@@ -616,7 +616,7 @@ int sem_abc_bptt(sem_abc *a, int n_steps, int n_roi, const int64_t *roi_nodes, c
         if (e == cudaSuccess) e = cudaMemcpy(nodes.data(), a->d_nodes, nb * 8, cudaMemcpyDeviceToHost);
         std::vector<int> map(n_int, -1);
         for (int64_t i = 0; i < nb; i++) map[nodes[i]] = (int)i;
-        if (e == cudaSuccess) e = cudaMemcpy(sidx, map.data(), n_int * 4, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = upload(sidx, map.data(), n_int, st);
         std::fill(map.begin(), map.end(), -1);
         bool twice = false;
         for (int r = 0; r < n_roi; r++) {
@@ -625,12 +625,13 @@ int sem_abc_bptt(sem_abc *a, int n_steps, int n_roi, const int64_t *roi_nodes, c
         }
         if (!twice && n_roi > 0) {
             if (e == cudaSuccess) e = dalloc(&ridx, (size_t)n_int);
-            if (e == cudaSuccess) e = cudaMemcpy(ridx, map.data(), n_int * 4, cudaMemcpyHostToDevice);
+            if (e == cudaSuccess) e = upload(ridx, map.data(), n_int, st);
         }
     }
-    if (e == cudaSuccess && n_roi > 0) e = cudaMemcpy(droi, roi.data(), n_roi * 8, cudaMemcpyHostToDevice);
+    // (both outlive the copies: the call waits for its stream before it returns)
+    if (e == cudaSuccess && n_roi > 0) e = cudaMemcpyAsync(droi, roi.data(), (size_t)n_roi * 8, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess && n_roi > 0)
-        e = cudaMemcpy(dref, ref, (size_t)n_steps * n_roi * 4, cudaMemcpyHostToDevice);
+        e = cudaMemcpyAsync(dref, ref, (size_t)n_steps * n_roi * 4, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(rec, 0, 2 * n_int * 4, st);  // p^{-1} = p^0 = 0: from rest
     // forward, the levels after every step recorded (by a kernel: the chain of dependent launches
     // goes on)

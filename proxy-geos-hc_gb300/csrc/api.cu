@@ -219,15 +219,15 @@ int solver_set_raw_sources(sem_solver *s, int n_src, const int64_t *nodes, const
     if (n_src > 0) {
         CUDA_TRY(dalloc(&s->d_src_off, off.size()));
         CUDA_TRY(dalloc(&s->d_src_perm, n_src));
-        CUDA_TRY(cudaMemcpy(s->d_src_off, off.data(), off.size() * 4, cudaMemcpyHostToDevice));
-        CUDA_TRY(cudaMemcpy(s->d_src_perm, perm.data(), n_src * 4, cudaMemcpyHostToDevice));
+        CUDA_TRY(upload(s->d_src_off, off.data(), off.size(), s->stream));
+        CUDA_TRY(upload(s->d_src_perm, perm.data(), n_src, s->stream));
         CUDA_TRY(dalloc(&s->d_src_node, n_src));
         CUDA_TRY(dalloc(&s->d_src_coef, n_src));
-        CUDA_TRY(cudaMemcpy(s->d_src_node, nodes, n_src * 8, cudaMemcpyHostToDevice));
-        CUDA_TRY(cudaMemcpy(s->d_src_coef, coef, n_src * 4, cudaMemcpyHostToDevice));
+        CUDA_TRY(upload(s->d_src_node, nodes, n_src, s->stream));
+        CUDA_TRY(upload(s->d_src_coef, coef, n_src, s->stream));
         if (n_samples > 0) {
             CUDA_TRY(dalloc(&s->d_wavelet, (size_t)n_src * n_samples));
-            CUDA_TRY(cudaMemcpy(s->d_wavelet, wavelet, (size_t)n_src * n_samples * 4, cudaMemcpyHostToDevice));
+            CUDA_TRY(upload(s->d_wavelet, wavelet, (size_t)n_src * n_samples, s->stream));
         }
     }
     return SEM_OK;
@@ -422,7 +422,7 @@ int sem_mesh_create_box(int ex, int ey, int ez, float lx, float ly, float lz, in
     cudaError_t e = dalloc(&m->d_vel, m->box.n_elem);
     if (e == cudaSuccess) {
         std::vector<float> v(m->box.n_elem, 1500.0f);  // SEMmesh::getModel
-        e = cudaMemcpy(m->d_vel, v.data(), v.size() * sizeof(float), cudaMemcpyHostToDevice);
+        e = upload(m->d_vel, v.data(), v.size(), 0);
     }
     if (e != cudaSuccess) {
         dfree(m->d_vel);
@@ -487,7 +487,7 @@ int sem_model_set_element_velocity(sem_mesh *m, const float *vel)
         if (!(vel[e] > 0) || !std::isfinite(vel[e]))
             return fail(SEM_ERR_ARG, "velocities must be positive and finite (element " +
                                          std::to_string(e) + ")");
-    CUDA_TRY(cudaMemcpy(m->d_vel, vel, m->box.n_elem * sizeof(float), cudaMemcpyHostToDevice));
+    CUDA_TRY(upload(m->d_vel, vel, m->box.n_elem, 0));
     dfree(m->d_slow2);
     m->model_version++;
     return SEM_OK;
@@ -503,7 +503,7 @@ int sem_model_set_node_slowness2(sem_mesh *m, const float *s2)
             return fail(SEM_ERR_ARG, "squared slowness must be positive and finite");
     if (!m->d_slow2) {
         CUDA_TRY(dalloc(&m->d_slow2, m->box.n_int));
-        CUDA_TRY(cudaMemset(m->d_slow2, 0, m->box.n_int * 4));
+        CUDA_TRY(cudaMemsetAsync(m->d_slow2, 0, m->box.n_int * 4, 0));
     }
     CUDA_TRY(field_from_host(m->d_slow2, s2, m->box.nx, m->box.nxp, m->box.nz * m->box.ny, 0));
     m->model_version++;
@@ -566,16 +566,16 @@ int sem_solver_create(sem_mesh *m, float dt, sem_solver **out)
     if (e != cudaSuccess) return cleanup(SEM_ERR_CUDA, cudaGetErrorString(e));
     s->own_stream = true;
     for (auto &p : s->d_p)
-        if ((e = dalloc(&p, s->n_int)) != cudaSuccess || (e = cudaMemset(p, 0, s->n_int * 4)) != cudaSuccess)
+        if ((e = dalloc(&p, s->n_int)) != cudaSuccess || (e = cudaMemsetAsync(p, 0, s->n_int * 4, s->stream)) != cudaSuccess)
             return cleanup(SEM_ERR_OOM, std::string("pressure levels: ") + cudaGetErrorString(e));
-    if ((e = dalloc(&s->d_a, s->n_int)) != cudaSuccess || (e = cudaMemset(s->d_a, 0, s->n_int * 4)) != cudaSuccess)
+    if ((e = dalloc(&s->d_a, s->n_int)) != cudaSuccess || (e = cudaMemsetAsync(s->d_a, 0, s->n_int * 4, s->stream)) != cudaSuccess)
         return cleanup(SEM_ERR_OOM, std::string("mass coefficient: ") + cudaGetErrorString(e));
-    if ((e = dalloc(&s->d_ctr, 2)) != cudaSuccess || (e = cudaMemset(s->d_ctr, 0, 8)) != cudaSuccess)
+    if ((e = dalloc(&s->d_ctr, 2)) != cudaSuccess || (e = cudaMemsetAsync(s->d_ctr, 0, 8, s->stream)) != cudaSuccess)
         return cleanup(SEM_ERR_CUDA, cudaGetErrorString(e));
-    if ((e = dalloc(&s->d_status, 1)) != cudaSuccess || (e = cudaMemset(s->d_status, 0, 4)) != cudaSuccess)
+    if ((e = dalloc(&s->d_status, 1)) != cudaSuccess || (e = cudaMemsetAsync(s->d_status, 0, 4, s->stream)) != cudaSuccess)
         return cleanup(SEM_ERR_CUDA, cudaGetErrorString(e));
     if ((e = dalloc(&s->d_w, m->box.order + 1)) != cudaSuccess ||
-        (e = cudaMemcpy(s->d_w, m->gll.w, (m->box.order + 1) * sizeof(double), cudaMemcpyHostToDevice)) != cudaSuccess)
+        (e = upload(s->d_w, m->gll.w, m->box.order + 1, s->stream)) != cudaSuccess)
         return cleanup(SEM_ERR_CUDA, cudaGetErrorString(e));
     // element coefficient table: g_d * w_a * w_b per pencil
     {
@@ -586,7 +586,7 @@ int sem_solver_create(sem_mesh *m, float dt, sem_solver **out)
                 for (int a2 = 0; a2 < o1; a2++)
                     tab[d * np + a2 + o1 * b] = (float)(m->geo.g[d] * m->gll.w[a2] * m->gll.w[b]);
         if ((e = dalloc(&s->d_tab, tab.size())) != cudaSuccess ||
-            (e = cudaMemcpy(s->d_tab, tab.data(), tab.size() * 4, cudaMemcpyHostToDevice)) != cudaSuccess)
+            (e = upload(s->d_tab, tab.data(), tab.size(), s->stream)) != cudaSuccess)
             return cleanup(SEM_ERR_CUDA, cudaGetErrorString(e));
     }
     if ((e = element_kernel_setup()) != cudaSuccess || (e = stencil_kernel_setup()) != cudaSuccess)
@@ -690,9 +690,9 @@ int sem_solver_set_sponge_profile(sem_solver *s, const float *sx, const float *s
         CUDA_TRY(dalloc(&s->d_sy, b.ny));
         CUDA_TRY(dalloc(&s->d_sz, b.nz));
     }
-    CUDA_TRY(cudaMemcpy(s->d_sx, sx, b.nx * 4, cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(s->d_sy, sy, b.ny * 4, cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(s->d_sz, sz, b.nz * 4, cudaMemcpyHostToDevice));
+    CUDA_TRY(upload(s->d_sx, sx, b.nx, s->stream));
+    CUDA_TRY(upload(s->d_sy, sy, b.ny, s->stream));
+    CUDA_TRY(upload(s->d_sz, sz, b.nz, s->stream));
     s->h_sx.assign(sx, sx + b.nx);
     s->h_sy.assign(sy, sy + b.ny);
     s->h_sz.assign(sz, sz + b.nz);
@@ -777,8 +777,8 @@ int sem_solver_set_receiver_nodes(sem_solver *s, int n_rec, const int64_t *nodes
     if (n_rec > 0) {
         CUDA_TRY(dalloc(&s->d_rec_node, n_rec));
         CUDA_TRY(dalloc(&s->d_rec_perm, n_rec));
-        CUDA_TRY(cudaMemcpy(s->d_rec_node, sorted.data(), n_rec * 8, cudaMemcpyHostToDevice));
-        CUDA_TRY(cudaMemcpy(s->d_rec_perm, perm.data(), n_rec * 4, cudaMemcpyHostToDevice));
+        CUDA_TRY(upload(s->d_rec_node, sorted.data(), n_rec, s->stream));
+        CUDA_TRY(upload(s->d_rec_perm, perm.data(), n_rec, s->stream));
     }
     return SEM_OK;
     GUARD_END
@@ -821,7 +821,7 @@ int solver_prepare(sem_solver *s, int64_t n_new)
             std::vector<float> rows;
             reference_element_rows(m->gll, 0.5 * b.lx / b.ex, 0.5 * b.lz / b.ez, 0.5 * b.ly / b.ey, rows);
             CUDA_TRY(dalloc(&s->d_rtab, rows.size()));
-            CUDA_TRY(cudaMemcpy(s->d_rtab, rows.data(), rows.size() * 4, cudaMemcpyHostToDevice));
+            CUDA_TRY(upload(s->d_rtab, rows.data(), rows.size(), s->stream));
             solver_invalidate_graphs(s);
         }
         if (s->rounding == SEM_ROUNDING_REFERENCE && !m->d_slow2 && s->mref_version != m->model_version) {
@@ -843,7 +843,7 @@ int solver_prepare(sem_solver *s, int64_t n_new)
                 for (int64_t q : s->rec_sorted) off[q / kUpdateNodesPerBlock + 1]++;
                 for (int64_t b = 0; b < nb; b++) off[b + 1] += off[b];
                 CUDA_TRY(dalloc(&s->d_upd_rec_off, nb + 1));
-                CUDA_TRY(cudaMemcpy(s->d_upd_rec_off, off.data(), (nb + 1) * sizeof(int), cudaMemcpyHostToDevice));
+                CUDA_TRY(upload(s->d_upd_rec_off, off.data(), nb + 1, s->stream));
             }
             s->upd_rec_version = s->rec_version;
             solver_invalidate_graphs(s);
@@ -870,11 +870,11 @@ int solver_prepare(sem_solver *s, int64_t n_new)
         if (stencil_bind(*s->stencil, s->d_p[0], s->d_p[1], s->d_a) != 0)
             return fail(SEM_ERR_CUDA, "tensor-map encoding failed (driver entry point cuTensorMapEncodeTiled)");
         if (s->stencil->rec_version != s->rec_version) {
-            CUDA_TRY(stencil_set_receivers(*s->stencil, s->rec_sorted.data(), s->nrec, s->rec_version));
+            CUDA_TRY(stencil_set_receivers(*s->stencil, s->rec_sorted.data(), s->nrec, s->rec_version, s->stream));
             solver_invalidate_graphs(s);
         }
         if (s->stencil->src_version != s->src_version) {
-            CUDA_TRY(stencil_set_sources(*s->stencil, s->src_group, s->src_version));
+            CUDA_TRY(stencil_set_sources(*s->stencil, s->src_group, s->src_version, s->stream));
             solver_invalidate_graphs(s);
         }
     }

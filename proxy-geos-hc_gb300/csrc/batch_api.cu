@@ -106,8 +106,8 @@ cudaError_t set_chunk(sem_batch *b, int ychunk)
     StencilTables &t = *b->st;
     t.ychunk = std::max(1, std::min<int>(ychunk, (int)t.ny));
     t.grid[2] = (int)((t.ny + t.ychunk - 1) / t.ychunk);
-    cudaError_t e = stencil_set_receivers(t, b->rec_sorted.data(), b->nrec, b->rec_version);
-    return e == cudaSuccess ? stencil_set_sources(t, b->src_group, b->src_version) : e;
+    cudaError_t e = stencil_set_receivers(t, b->rec_sorted.data(), b->nrec, b->rec_version, b->stream);
+    return e == cudaSuccess ? stencil_set_sources(t, b->src_group, b->src_version, b->stream) : e;
 }
 
 int prepare(sem_batch *b, int64_t n_new)
@@ -121,11 +121,11 @@ int prepare(sem_batch *b, int64_t n_new)
     if (stencil_bind(*b->st, b->d_p[0], b->d_p[1], b->d_a) != 0)
         return sem_fail(SEM_ERR_CUDA, "tensor-map encoding failed (driver entry point cuTensorMapEncodeTiled)");
     if (b->st->rec_version != b->rec_version) {
-        CUDA_TRY(stencil_set_receivers(*b->st, b->rec_sorted.data(), b->nrec, b->rec_version));
+        CUDA_TRY(stencil_set_receivers(*b->st, b->rec_sorted.data(), b->nrec, b->rec_version, b->stream));
         invalidate(b);
     }
     if (b->st->src_version != b->src_version) {
-        CUDA_TRY(stencil_set_sources(*b->st, b->src_group, b->src_version));
+        CUDA_TRY(stencil_set_sources(*b->st, b->src_group, b->src_version, b->stream));
         invalidate(b);
     }
     if (b->nrec > 0 && b->steps_done + n_new > b->trace_cap) {
@@ -204,16 +204,16 @@ int sem_batch_create(sem_mesh *m, float dt, int n_shots, sem_batch **out)
     b->own_stream = true;
     const size_t n = (size_t)b->n_int * b->nshot;
     for (auto &p : b->d_p)
-        if ((e = dalloc(&p, n)) != cudaSuccess || (e = cudaMemset(p, 0, n * 4)) != cudaSuccess)
+        if ((e = dalloc(&p, n)) != cudaSuccess || (e = cudaMemsetAsync(p, 0, n * 4, b->stream)) != cudaSuccess)
             return cleanup(SEM_ERR_OOM, std::string("pressure levels: ") + cudaGetErrorString(e));
-    if ((e = dalloc(&b->d_a, b->n_int)) != cudaSuccess || (e = cudaMemset(b->d_a, 0, b->n_int * 4)) != cudaSuccess)
+    if ((e = dalloc(&b->d_a, b->n_int)) != cudaSuccess || (e = cudaMemsetAsync(b->d_a, 0, b->n_int * 4, b->stream)) != cudaSuccess)
         return cleanup(SEM_ERR_OOM, cudaGetErrorString(e));
-    if ((e = dalloc(&b->d_ctr, 2)) != cudaSuccess || (e = cudaMemset(b->d_ctr, 0, 8)) != cudaSuccess)
+    if ((e = dalloc(&b->d_ctr, 2)) != cudaSuccess || (e = cudaMemsetAsync(b->d_ctr, 0, 8, b->stream)) != cudaSuccess)
         return cleanup(SEM_ERR_CUDA, cudaGetErrorString(e));
-    if ((e = dalloc(&b->d_status, 1)) != cudaSuccess || (e = cudaMemset(b->d_status, 0, 4)) != cudaSuccess)
+    if ((e = dalloc(&b->d_status, 1)) != cudaSuccess || (e = cudaMemsetAsync(b->d_status, 0, 4, b->stream)) != cudaSuccess)
         return cleanup(SEM_ERR_CUDA, cudaGetErrorString(e));
     if ((e = dalloc(&b->d_w, m->box.order + 1)) != cudaSuccess ||
-        (e = cudaMemcpy(b->d_w, m->gll.w, (m->box.order + 1) * sizeof(double), cudaMemcpyHostToDevice)) != cudaSuccess)
+        (e = upload(b->d_w, m->gll.w, m->box.order + 1, b->stream)) != cudaSuccess)
         return cleanup(SEM_ERR_CUDA, cudaGetErrorString(e));
     if ((e = stencil_kernel_setup()) != cudaSuccess) return cleanup(SEM_ERR_CUDA, std::string("kernel set-up: ") + cudaGetErrorString(e));
     if (stencil_tables_create(m->box, m->gll, m->geo, n_shots, &b->st, kTileDefault) != 0) return cleanup(SEM_ERR_CUDA, "stencil tables");
@@ -253,9 +253,9 @@ int sem_batch_set_sponge_profile(sem_batch *b, const float *sx, const float *sy,
         CUDA_TRY(dalloc(&b->d_sy, x.ny));
         CUDA_TRY(dalloc(&b->d_sz, x.nz));
     }
-    CUDA_TRY(cudaMemcpy(b->d_sx, sx, x.nx * 4, cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(b->d_sy, sy, x.ny * 4, cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(b->d_sz, sz, x.nz * 4, cudaMemcpyHostToDevice));
+    CUDA_TRY(upload(b->d_sx, sx, x.nx, b->stream));
+    CUDA_TRY(upload(b->d_sy, sy, x.ny, b->stream));
+    CUDA_TRY(upload(b->d_sz, sz, x.nz, b->stream));
     b->sponge = true;
     return SEM_OK;
     GUARD_END
@@ -300,17 +300,17 @@ int sem_batch_set_sources(sem_batch *b, const int64_t *elements, const float *wa
         const int off[2] = {0, 1}, perm[1] = {0};
         CUDA_TRY(dalloc(&b->d_src_off, 2));
         CUDA_TRY(dalloc(&b->d_src_perm, 1));
-        CUDA_TRY(cudaMemcpy(b->d_src_off, off, sizeof(off), cudaMemcpyHostToDevice));
-        CUDA_TRY(cudaMemcpy(b->d_src_perm, perm, sizeof(perm), cudaMemcpyHostToDevice));
+        CUDA_TRY(upload(b->d_src_off, off, 2, b->stream));
+        CUDA_TRY(upload(b->d_src_perm, perm, 1, b->stream));
         b->src_group.push_back(node[0]);
     }
     CUDA_TRY(dalloc(&b->d_src_node, b->nshot));
     CUDA_TRY(dalloc(&b->d_src_coef, b->nshot));
-    CUDA_TRY(cudaMemcpy(b->d_src_node, node.data(), b->nshot * 8, cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(b->d_src_coef, coef.data(), b->nshot * 4, cudaMemcpyHostToDevice));
+    CUDA_TRY(upload(b->d_src_node, node.data(), b->nshot, b->stream));
+    CUDA_TRY(upload(b->d_src_coef, coef.data(), b->nshot, b->stream));
     if (n_samples > 0) {
         CUDA_TRY(dalloc(&b->d_wavelet, (size_t)b->nshot * n_samples));
-        CUDA_TRY(cudaMemcpy(b->d_wavelet, wavelet, (size_t)b->nshot * n_samples * 4, cudaMemcpyHostToDevice));
+        CUDA_TRY(upload(b->d_wavelet, wavelet, (size_t)b->nshot * n_samples, b->stream));
     }
     b->nsamples = n_samples;
     return SEM_OK;
@@ -352,8 +352,8 @@ int sem_batch_set_receiver_nodes(sem_batch *b, int n_rec, const int64_t *nodes)
     if (n_rec > 0) {
         CUDA_TRY(dalloc(&b->d_rec_node, n_rec));
         CUDA_TRY(dalloc(&b->d_rec_perm, n_rec));
-        CUDA_TRY(cudaMemcpy(b->d_rec_node, sorted.data(), n_rec * 8, cudaMemcpyHostToDevice));
-        CUDA_TRY(cudaMemcpy(b->d_rec_perm, perm.data(), n_rec * 4, cudaMemcpyHostToDevice));
+        CUDA_TRY(upload(b->d_rec_node, sorted.data(), n_rec, b->stream));
+        CUDA_TRY(upload(b->d_rec_perm, perm.data(), n_rec, b->stream));
     }
     return SEM_OK;
     GUARD_END

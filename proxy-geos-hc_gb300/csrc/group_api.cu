@@ -243,9 +243,9 @@ int write_descriptors(sem_group *g)
         return sem_fail(SEM_ERR_STATE, "group launch changed size");
     }
     g->n_ctas = (int)cta_member.size();
-    // the group stream is idle here (callers synchronise it first), so plain copies are ordered
-    CUDA_TRY(cudaMemcpy(g->d_mem, h.data(), n * sizeof(GroupMember), cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(g->d_cta_member, cta_member.data(), cta_member.size() * sizeof(int), cudaMemcpyHostToDevice));
+    // (the group stream is idle here: callers synchronise it first)
+    CUDA_TRY(semgb::upload(g->d_mem, h.data(), n, g->stream));
+    CUDA_TRY(semgb::upload(g->d_cta_member, cta_member.data(), cta_member.size(), g->stream));
     return SEM_OK;
 }
 
@@ -277,14 +277,14 @@ int build_one_launch(sem_group *g)
             return sem_fail(SEM_ERR_CUDA, "tensor-map encoding failed (driver entry point cuTensorMapEncodeTiled)");
         t->ychunk = chunks[i];
         t->grid[2] = (int)((t->ny + chunks[i] - 1) / chunks[i]);
-        CUDA_TRY(semgb::stencil_set_receivers(*t, s->rec_sorted.data(), s->nrec, s->rec_version));
-        CUDA_TRY(semgb::stencil_set_sources(*t, s->src_group, s->src_version));
+        CUDA_TRY(semgb::stencil_set_receivers(*t, s->rec_sorted.data(), s->nrec, s->rec_version, g->stream));
+        CUDA_TRY(semgb::stencil_set_sources(*t, s->src_group, s->src_version, g->stream));
         if (!s->sponge && !g->ones[i]) {
             const Box &b = s->mesh->box;
             const size_t len = (size_t)std::max(b.nx, std::max(b.ny, b.nz));
             std::vector<float> one(len, 1.f);
             CUDA_TRY(cudaMalloc(&g->ones[i], len * sizeof(float)));
-            CUDA_TRY(cudaMemcpy(g->ones[i], one.data(), len * sizeof(float), cudaMemcpyHostToDevice));
+            CUDA_TRY(semgb::upload(g->ones[i], one.data(), len, g->stream));
         }
     }
     g->max_order = max_order;

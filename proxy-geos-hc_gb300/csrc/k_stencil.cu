@@ -365,7 +365,8 @@ static int64_t owner_cta(const StencilTables &t, int64_t n)
     return bx + t.grid[0] * (bz + t.grid[1] * (int64_t)chunk);
 }
 
-cudaError_t stencil_set_receivers(StencilTables &t, const int64_t *sorted_nodes, int nrec, uint64_t version)
+cudaError_t stencil_set_receivers(StencilTables &t, const int64_t *sorted_nodes, int nrec, uint64_t version,
+                                  cudaStream_t stream)
 {
     if (t.d_rec_off) { cudaFree(t.d_rec_off); t.d_rec_off = nullptr; }
     if (t.d_rec_idx) { cudaFree(t.d_rec_idx); t.d_rec_idx = nullptr; }
@@ -384,12 +385,13 @@ cudaError_t stencil_set_receivers(StencilTables &t, const int64_t *sorted_nodes,
     cudaError_t e;
     if ((e = cudaMalloc(&t.d_rec_off, (ncta + 1) * sizeof(int))) != cudaSuccess) return e;
     if ((e = cudaMalloc(&t.d_rec_idx, nrec * sizeof(int))) != cudaSuccess) return e;
-    if ((e = cudaMemcpy(t.d_rec_off, count.data(), (ncta + 1) * sizeof(int), cudaMemcpyHostToDevice)) != cudaSuccess)
+    if ((e = upload(t.d_rec_off, count.data(), ncta + 1, stream)) != cudaSuccess)
         return e;
-    return cudaMemcpy(t.d_rec_idx, idx.data(), nrec * sizeof(int), cudaMemcpyHostToDevice);
+    return upload(t.d_rec_idx, idx.data(), nrec, stream);
 }
 
-cudaError_t stencil_set_sources(StencilTables &t, const std::vector<int64_t> &group_nodes, uint64_t version)
+cudaError_t stencil_set_sources(StencilTables &t, const std::vector<int64_t> &group_nodes, uint64_t version,
+                                cudaStream_t stream)
 {
     if (t.d_src_cta) { cudaFree(t.d_src_cta); t.d_src_cta = nullptr; }
     t.src_version = version;
@@ -398,7 +400,7 @@ cudaError_t stencil_set_sources(StencilTables &t, const std::vector<int64_t> &gr
     for (size_t u = 0; u < cta.size(); u++) cta[u] = (int)owner_cta(t, group_nodes[u]);
     cudaError_t e = cudaMalloc(&t.d_src_cta, cta.size() * sizeof(int));
     if (e != cudaSuccess) return e;
-    return cudaMemcpy(t.d_src_cta, cta.data(), cta.size() * sizeof(int), cudaMemcpyHostToDevice);
+    return upload(t.d_src_cta, cta.data(), cta.size(), stream);
 }
 
 int stencil_set_class_table(StencilTables &t, const float *tab)

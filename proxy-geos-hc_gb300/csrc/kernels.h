@@ -15,6 +15,16 @@
 
 namespace semgb {
 
+// A host array to the device on the stream whose work reads it, landed when this returns.  A plain cudaMemcpy
+// from pageable memory may return before its transfer has, and like a plain cudaMemset it runs on the
+// default stream, which the solvers' non-blocking streams do not wait for.
+template <class T>
+inline cudaError_t upload(T *dst, const T *src, size_t n, cudaStream_t s)
+{
+    cudaError_t e = cudaMemcpyAsync(dst, src, n * sizeof(T), cudaMemcpyHostToDevice, s);
+    return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
+}
+
 // Uniform-box geometry: J = diag(hx/2, hz/2, hy/2) for the reference directions
 // (xi1 -> x, xi2 -> z, xi3 -> y).  g[d] = |detJ| / J_dd^2 (the diagonal of B, SEMQkGLIntegrals
 // .hpp:344-349); off-diagonal terms are exactly zero on this mesh.

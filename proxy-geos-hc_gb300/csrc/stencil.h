@@ -157,10 +157,12 @@ int stencil_tables_create(const Box &b, const Gll &g, const Geometry &geo, int n
 void stencil_tile_dims(int order, int shape, int &tx, int &tz, int &hx, int &threads);
 // Describe the solver's two pressure buffers and its dt^2/M buffer with tensor maps.
 int stencil_bind(StencilTables &t, const float *p0, const float *p1, const float *a);
-// Group node-sorted receivers (device-layout indices) by owning CTA (device CSR in t).
-cudaError_t stencil_set_receivers(StencilTables &t, const int64_t *sorted_nodes, int nrec, uint64_t version);
+// Group node-sorted receivers (device-layout indices) by owning CTA (device CSR in t, uploaded on `stream`).
+cudaError_t stencil_set_receivers(StencilTables &t, const int64_t *sorted_nodes, int nrec, uint64_t version,
+                                  cudaStream_t stream);
 // Owning CTA of each source group (group_nodes: its node, device layout), for StencilArgs::src_cta.
-cudaError_t stencil_set_sources(StencilTables &t, const std::vector<int64_t> &group_nodes, uint64_t version);
+cudaError_t stencil_set_sources(StencilTables &t, const std::vector<int64_t> &group_nodes, uint64_t version,
+                                cudaStream_t stream);
 // Switch the pass to the reference-rounding operator with node-class table `tab` (layout of
 // reference_class_table, copied), or back to the tensor-product operator (tab null).
 int stencil_set_class_table(StencilTables &t, const float *tab);

@@ -826,7 +826,8 @@ cudaError_t upload_stencil_constants()
     std::vector<float2> all2(all.size());
     for (size_t i = 0; i < all.size(); i++) all2[i] = make_float2(all[i], all[i]);
     if ((e = cudaMemcpyToSymbol(c_T2, all2.data(), all2.size() * sizeof(float2))) != cudaSuccess) return e;
-    return cudaMemcpyToSymbol(c_wa, wa.data(), wa.size() * sizeof(float));
+    if ((e = cudaMemcpyToSymbol(c_wa, wa.data(), wa.size() * sizeof(float))) != cudaSuccess) return e;
+    return cudaStreamSynchronize(0);  // landed (copied on the default stream) before any stream's kernels read them
 }
 
 }  // namespace

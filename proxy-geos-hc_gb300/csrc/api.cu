@@ -461,8 +461,14 @@ static int ensure_conn(sem_mesh *m, cudaStream_t s)
     if (m->d_conn) return SEM_OK;
     if (m->box.n_int > 0x7fffffffLL)
         return fail(SEM_ERR_ARG, "element kernel needs fewer than 2^31 nodes (int32 connectivity)");
-    CUDA_TRY(dalloc(&m->d_conn, (size_t)m->box.n_elem * m->box.npe));
-    CUDA_TRY(launch_connectivity(m->d_conn, m->box.ex, m->box.ey, m->box.ez, m->box.order, m->box.nxp, s));
+    int32_t *conn = nullptr;
+    CUDA_TRY(dalloc(&conn, (size_t)m->box.n_elem * m->box.npe));
+    cudaError_t e = launch_connectivity(conn, m->box.ex, m->box.ey, m->box.ez, m->box.order, m->box.nxp, s);
+    // the mesh's other solvers, on their own streams, take the map as it stands: filled before it is theirs
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) dfree(conn);
+    CUDA_TRY(e);
+    m->d_conn = conn;
     return SEM_OK;
 }
 

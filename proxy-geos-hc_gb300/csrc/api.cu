@@ -493,6 +493,8 @@ int sem_model_set_element_velocity(sem_mesh *m, const float *vel)
         if (!(vel[e] > 0) || !std::isfinite(vel[e]))
             return fail(SEM_ERR_ARG, "velocities must be positive and finite (element " +
                                          std::to_string(e) + ")");
+    // runs under way form their mass from the old model, on streams that the upload does not wait for
+    CUDA_TRY(cudaDeviceSynchronize());
     CUDA_TRY(upload(m->d_vel, vel, m->box.n_elem, 0));
     dfree(m->d_slow2);
     m->model_version++;
@@ -507,6 +509,7 @@ int sem_model_set_node_slowness2(sem_mesh *m, const float *s2)
     for (int64_t i = 0; i < m->box.n_nodes; i++)
         if (!(s2[i] > 0) || !std::isfinite(s2[i]))
             return fail(SEM_ERR_ARG, "squared slowness must be positive and finite");
+    CUDA_TRY(cudaDeviceSynchronize());  // as sem_model_set_element_velocity
     if (!m->d_slow2) {
         CUDA_TRY(dalloc(&m->d_slow2, m->box.n_int));
         CUDA_TRY(cudaMemsetAsync(m->d_slow2, 0, m->box.n_int * 4, 0));

@@ -33,8 +33,9 @@ void solver_invalidate_graphs(sem_solver *s)
 {
     s->plain_runs = 0;
     s->graph_gen++;
-    for (auto &g : s->graph)
-        if (g) { cudaGraphExecDestroy(g); g = nullptr; }
+    for (auto *gs : {s->graph, s->pair})
+        for (int c = 0; c < 2; c++)
+            if (gs[c]) { cudaGraphExecDestroy(gs[c]); gs[c] = nullptr; }
 }
 
 namespace {
@@ -1009,24 +1010,48 @@ cudaError_t solver_enqueue_run(sem_solver *s, int c, int n, const std::function<
 
 extern "C" {
 
-static int build_graph(sem_solver *s, int c)
+// n steps from level c as a graph
+static int build_graph(sem_solver *s, int c, int n, cudaGraphExec_t &out)
 {
     cudaGraph_t g = nullptr;
     CUDA_TRY(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-    cudaError_t e2 = solver_enqueue_run(s, c, kGraphSteps);
+    cudaError_t e2 = solver_enqueue_run(s, c, n);
     cudaError_t e3 = cudaStreamEndCapture(s->stream, &g);
     if (e2 != cudaSuccess || e3 != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
         return fail(SEM_ERR_CUDA, std::string("graph capture: ") +
                                       cudaGetErrorString(e2 != cudaSuccess ? e2 : e3));
     }
-    cudaError_t e4 = cudaGraphInstantiate(&s->graph[c], g, 0);
+    cudaError_t e4 = cudaGraphInstantiate(&out, g, 0);
     cudaGraphDestroy(g);
     if (e4 != cudaSuccess) return fail(SEM_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e4));
     return SEM_OK;
 }
 
 static constexpr int kPlainRuns = 8;  // runs of kGraphSteps launched before a graph is made
+
+// n steps from the current level outside the graphs of kGraphSteps
+static int enqueue_steps(sem_solver *s, int n)
+{
+    int done = 0;
+    // The element path launches three kernels a step, which cost the host more than a small box's take:
+    // pairs of steps from a graph.  Launched -> pairs, per step: 8^3 and 12^3 elements of order 2 12.6 ->
+    // 7.5 us, 40^3 17.7 -> 12.6, 24^3 of order 4 22.8 -> 17.5.  (A run of passes is one launch a step: launched
+    // 4.3 to 5.4 us, pairs 5.4.)
+    if (resolved_kernel(s) == SEM_KERNEL_ELEMENT) {
+        for (; n - done >= 2; done += 2) {
+            cudaGraphExec_t &ge = s->pair[s->cur];
+            if (!ge) {
+                int rc = build_graph(s, s->cur, 2, ge);
+                if (rc) return rc;
+            }
+            CUDA_TRY(cudaGraphLaunch(ge, s->stream));
+        }
+    }
+    if (done < n) CUDA_TRY(solver_enqueue_run(s, s->cur, n - done));
+    s->cur ^= n & 1;
+    return SEM_OK;
+}
 
 int sem_solver_step(sem_solver *s, int n_steps)
 {
@@ -1038,25 +1063,22 @@ int sem_solver_step(sem_solver *s, int n_steps)
     if (rc) return rc;
     int done = 0;
     for (; n_steps - done >= kGraphSteps; done += kGraphSteps) {  // an even number of swaps
-        // Few steps since the last change (sources, receivers, model): launched one by one.  Capturing and
+        // Few steps since the last change (sources, receivers, model): enqueue_steps, launched.  Capturing and
         // instantiating takes 55 us and replaying saves at most 0.25 us a step: the first 16 steps after a
         // change, graph -> launches, 12^3 elements of order 2 160 -> 103 us, 24^3 of order 4 231 -> 176, 40^3
         // 400 -> 346; 128 steps 638 -> 597, 1200 -> 1173, 2550 -> 2514; beyond, the host's time counts.
         if (!s->graph[s->cur] && s->plain_runs + (n_steps - done) / kGraphSteps <= kPlainRuns) {
-            CUDA_TRY(solver_enqueue_run(s, s->cur, kGraphSteps));
+            if ((rc = enqueue_steps(s, kGraphSteps)) != SEM_OK) return rc;
             s->plain_runs++;
             continue;
         }
         if (!s->graph[s->cur]) {
-            rc = build_graph(s, s->cur);
+            rc = build_graph(s, s->cur, kGraphSteps, s->graph[s->cur]);
             if (rc) return rc;
         }
         CUDA_TRY(cudaGraphLaunch(s->graph[s->cur], s->stream));
     }
-    if (done < n_steps) {
-        CUDA_TRY(solver_enqueue_run(s, s->cur, n_steps - done));
-        s->cur ^= (n_steps - done) & 1;
-    }
+    if ((rc = enqueue_steps(s, n_steps - done)) != SEM_OK) return rc;
     s->steps_done += n_steps;
     return SEM_OK;
     GUARD_END

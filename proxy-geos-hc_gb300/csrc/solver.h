@@ -69,7 +69,8 @@ struct sem_solver {
     int64_t steps_done = 0;
     // graphs: [parity] kGraphSteps steps starting at level `parity`
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
-    int plain_runs = 0;  // runs of kGraphSteps enqueued without a graph since the last change
+    cudaGraphExec_t pair[2] = {nullptr, nullptr};  // two steps of the element path
+    int plain_runs = 0;  // runs of kGraphSteps enqueued without their graph since the last change
     uint64_t graph_gen = 0;  // bumped whenever captured launch parameters may have changed
 };
 

@@ -116,3 +116,23 @@ def test_group_run_equals_solo_single_steps(semgb_lib, cuda_device, launch):
         for m, s in members + solo:
             s.close()
             m.close()
+
+
+@pytest.mark.parametrize("calls", [[1], [2], [3], [15], [16], [17], [33], [16] * 9 + [3], [145, 18]])
+def test_element_run_equals_single_steps(semgb_lib, cuda_device, calls):
+    """The element path's steps: alone, in pairs and in runs of 16 replayed from graphs.  Its float atomics add
+    the eight or fewer contributions of a node in any order: a few units in the last place per step."""
+    semgb = semgb_lib
+    ex, ey, ez, order = 7, 8, 6, 3
+    el, n = _elements(ex, ey, ez), sum(calls)
+    m1, a = _solver(semgb, ex, ey, ez, order, el, n, "element")
+    m2, b = _solver(semgb, ex, ey, ez, order, el, n, "element")
+    for c in calls:
+        a.step(c)
+    for _ in range(n):
+        b.step(1)
+    for x, y in ((a.traces(), b.traces()), (a.pressure(), b.pressure()), (a.pressure(1), b.pressure(1))):
+        assert np.abs(x - y).max() <= 1e-5 * np.abs(y).max()
+    assert np.abs(a.pressure()).max() > 0
+    for x in (a, b, m1, m2):
+        x.close()

@@ -32,6 +32,7 @@ struct sem_group {
     int want = SEM_GROUP_ONE_LAUNCH;   // requested launch form
     int form = -1;                     // form of the graphs and state below
     cudaGraphExec_t graph[2] = {nullptr, nullptr};  // [f]: kGraphSteps steps starting at parity f
+    cudaGraphExec_t pair[2] = {nullptr, nullptr};   // [f]: two steps as branches
     std::vector<uint64_t> gen;         // members' graph generations at build
     std::vector<int> cur0;             // member's current level at parity 0
     int flip = 0;                      // parity of the next step
@@ -47,8 +48,9 @@ namespace {
 
 void drop_graphs(sem_group *g)
 {
-    for (auto &x : g->graph)
-        if (x) { cudaGraphExecDestroy(x); x = nullptr; }
+    for (auto *gs : {g->graph, g->pair})
+        for (int f = 0; f < 2; f++)
+            if (gs[f]) { cudaGraphExecDestroy(gs[f]); gs[f] = nullptr; }
 }
 
 void free_one_launch(sem_group *g)
@@ -113,18 +115,18 @@ cudaError_t enqueue(sem_group *g, int steps, int parity)
     return g->form == SEM_GROUP_ONE_LAUNCH ? enqueue_one_launch(g, steps, parity) : enqueue_branches(g, steps, parity);
 }
 
-int capture(sem_group *g, int parity)
+int capture(sem_group *g, int steps, int parity, cudaGraphExec_t &out)
 {
     cudaGraph_t graph = nullptr;
     CUDA_TRY(cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal));
-    cudaError_t e1 = enqueue(g, kGraphSteps, parity);
+    cudaError_t e1 = enqueue(g, steps, parity);
     cudaError_t e2 = cudaStreamEndCapture(g->stream, &graph);
     if (e1 != cudaSuccess || e2 != cudaSuccess) {
         if (graph) cudaGraphDestroy(graph);
         return sem_fail(SEM_ERR_CUDA, std::string("group graph capture: ") +
                                           cudaGetErrorString(e1 != cudaSuccess ? e1 : e2));
     }
-    cudaError_t e3 = cudaGraphInstantiate(&g->graph[parity], graph, 0);
+    cudaError_t e3 = cudaGraphInstantiate(&out, graph, 0);
     cudaGraphDestroy(graph);
     if (e3 != cudaSuccess) return sem_fail(SEM_ERR_CUDA, cudaGetErrorString(e3));
     return SEM_OK;
@@ -397,10 +399,23 @@ int sem_group_step(sem_group *g, int n_steps)
     int done = 0;
     for (; n_steps - done >= kGraphSteps; done += kGraphSteps) {
         if (!g->graph[g->flip]) {
-            int rc = capture(g, g->flip);
+            int rc = capture(g, kGraphSteps, g->flip, g->graph[g->flip]);
             if (rc) return rc;
         }
         CUDA_TRY(cudaGraphLaunch(g->graph[g->flip], g->stream));
+    }
+    // Few steps left of many branches: the forks, joins and launches of a member cost the host more than replaying
+    // pairs of steps.  32 members of 8 to 24 elements, launched -> pairs, us a step: 2 a call 130 -> 98, 3 a
+    // call 109 -> 101, 4 a call 101 and 122 (two runs) -> 104, but 6 a call 110 against 106 and 8 a call 96 against
+    // 103; 8 members of 24 to 40 elements, 2 a call 46.9 against 48.8.
+    if (form == SEM_GROUP_BRANCHES && n > 16 && n_steps - done < 5) {
+        for (; n_steps - done >= 2; done += 2) {
+            if (!g->pair[g->flip]) {
+                int rc = capture(g, 2, g->flip, g->pair[g->flip]);
+                if (rc) return rc;
+            }
+            CUDA_TRY(cudaGraphLaunch(g->pair[g->flip], g->stream));
+        }
     }
     if (done < n_steps) {
         CUDA_TRY(enqueue(g, n_steps - done, g->flip));

@@ -136,3 +136,27 @@ def test_element_run_equals_single_steps(semgb_lib, cuda_device, calls):
     assert np.abs(a.pressure()).max() > 0
     for x in (a, b, m1, m2):
         x.close()
+
+
+@pytest.mark.parametrize("members", [16, 17])
+def test_branches_of_few_steps_equal_solo_single_steps(semgb_lib, cuda_device, members):
+    """Calls of two to four steps, which more than 16 branches replay in pairs, from both parities, and of five."""
+    semgb = semgb_lib
+    boxes = [(3 + i % 4, 4, 3 + i % 3, 1 + i % 4) for i in range(members)]
+    calls = [2, 3, 2, 1, 3, 4, 5, 18, 20, 21]
+    n = sum(calls)
+    grouped = [_solver(semgb, ex, ey, ez, o, _elements(ex, ey, ez) % (ex * ey * ez), n) for ex, ey, ez, o in boxes]
+    solo = [_solver(semgb, ex, ey, ez, o, _elements(ex, ey, ez) % (ex * ey * ez), n) for ex, ey, ez, o in boxes]
+    g = semgb.Group([s for _, s in grouped], semgb.GROUP_BRANCHES)
+    for c in calls:
+        g.step(c)
+    g.synchronize()
+    for (_, a), (_, b) in zip(grouped, solo):
+        for _ in range(n):
+            b.step(1)
+        assert np.array_equal(a.traces(), b.traces()) and np.array_equal(a.pressure(), b.pressure())
+        assert np.abs(b.traces()).max() > 0
+    g.close()
+    for m, s in grouped + solo:
+        s.close()
+        m.close()

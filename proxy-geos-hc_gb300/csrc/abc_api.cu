@@ -58,6 +58,7 @@ struct sem_abc {
     // parity; valid while the solver's captured parameters are (graph_gen)
     cudaGraphExec_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
     uint64_t graph_gen = 0;
+    int plain_runs = 0;  // runs of kGraphSteps launched since the graphs were dropped
     float *hist_now() const { return face && hcur ? d_hist_alt : d_hist; }
     float *hist_next() const { return face && !hcur ? d_hist_alt : d_hist; }
 };
@@ -533,10 +534,18 @@ int sem_abc_step(sem_abc *a, int n_steps)
             for (auto &g : row)
                 if (g) { cudaGraphExecDestroy(g); g = nullptr; }
         a->graph_gen = s->graph_gen;
+        a->plain_runs = 0;
     }
     int done = 0;
     for (; n_steps - done >= kGraphSteps; done += kGraphSteps) {
         cudaGraphExec_t &ge = a->graph[s->cur][a->hcur];
+        if (!ge && a->plain_runs + (n_steps - done) / kGraphSteps <= kPlainRuns) {
+            // (first 16 steps, graph -> launches: 8^3 elements of order 4 357 -> 240 us, 24^3 514 -> 386; 128 steps
+            // 1703 -> 1728, 2932 -> 2897)
+            CUDA_TRY(enqueue_corrected(a, kGraphSteps));
+            a->plain_runs++;
+            continue;
+        }
         if (!ge) {
             // an even number of steps: the level and history parities come back to where they
             // started

@@ -1028,8 +1028,6 @@ static int build_graph(sem_solver *s, int c, int n, cudaGraphExec_t &out)
     return SEM_OK;
 }
 
-static constexpr int kPlainRuns = 8;  // runs of kGraphSteps launched before a graph is made
-
 // n steps from the current level outside the graphs of kGraphSteps
 static int enqueue_steps(sem_solver *s, int n)
 {
@@ -1063,10 +1061,6 @@ int sem_solver_step(sem_solver *s, int n_steps)
     if (rc) return rc;
     int done = 0;
     for (; n_steps - done >= kGraphSteps; done += kGraphSteps) {  // an even number of swaps
-        // Few steps since the last change (sources, receivers, model): enqueue_steps, launched.  Capturing and
-        // instantiating takes 55 us and replaying saves at most 0.25 us a step: the first 16 steps after a
-        // change, graph -> launches, 12^3 elements of order 2 160 -> 103 us, 24^3 of order 4 231 -> 176, 40^3
-        // 400 -> 346; 128 steps 638 -> 597, 1200 -> 1173, 2550 -> 2514; beyond, the host's time counts.
         if (!s->graph[s->cur] && s->plain_runs + (n_steps - done) / kGraphSteps <= kPlainRuns) {
             if ((rc = enqueue_steps(s, kGraphSteps)) != SEM_OK) return rc;
             s->plain_runs++;

@@ -54,12 +54,14 @@ struct sem_batch {
     BatchTuning tune;
     bool tuned = false;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};  // [parity] kGraphSteps steps
+    int plain_runs = 0;  // runs of kGraphSteps launched since the graphs were dropped
 };
 
 namespace {
 
 void invalidate(sem_batch *b)
 {
+    b->plain_runs = 0;
     for (auto &g : b->graph)
         if (g) { cudaGraphExecDestroy(g); g = nullptr; }
 }
@@ -379,6 +381,13 @@ int sem_batch_step(sem_batch *b, int n_steps)
     if (rc) return rc;
     int done = 0;
     for (; n_steps - done >= kGraphSteps; done += kGraphSteps) {
+        if (!b->graph[b->cur] && b->plain_runs + (n_steps - done) / kGraphSteps <= kPlainRuns) {
+            // (first 16 steps of 8 shots, graph -> launches: 8^3 elements of order 4 180 -> 119 us, 16^3 239 ->
+            // 180; 128 steps 808 -> 780, 1270 -> 1253)
+            CUDA_TRY(enqueue(b, b->cur, kGraphSteps));
+            b->plain_runs++;
+            continue;
+        }
         if (!b->graph[b->cur]) {
             cudaGraph_t g = nullptr;
             CUDA_TRY(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));

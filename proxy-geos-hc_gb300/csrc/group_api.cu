@@ -33,6 +33,7 @@ struct sem_group {
     int form = -1;                     // form of the graphs and state below
     cudaGraphExec_t graph[2] = {nullptr, nullptr};  // [f]: kGraphSteps steps starting at parity f
     cudaGraphExec_t pair[2] = {nullptr, nullptr};   // [f]: two steps as branches
+    int plain_runs = 0;                // runs of kGraphSteps launched since the graphs were dropped
     std::vector<uint64_t> gen;         // members' graph generations at build
     std::vector<int> cur0;             // member's current level at parity 0
     int flip = 0;                      // parity of the next step
@@ -46,8 +47,11 @@ struct sem_group {
 
 namespace {
 
+constexpr int kPlainBranchRuns = 4;  // as kPlainRuns, of the branches form
+
 void drop_graphs(sem_group *g)
 {
+    g->plain_runs = 0;
     for (auto *gs : {g->graph, g->pair})
         for (int f = 0; f < 2; f++)
             if (gs[f]) { cudaGraphExecDestroy(gs[f]); gs[f] = nullptr; }
@@ -398,6 +402,15 @@ int sem_group_step(sem_group *g, int n_steps)
     }
     int done = 0;
     for (; n_steps - done >= kGraphSteps; done += kGraphSteps) {
+        if (form == SEM_GROUP_BRANCHES && !g->graph[g->flip] &&
+            g->plain_runs + (n_steps - done) / kGraphSteps <= kPlainBranchRuns) {
+            // (first 16 steps, graph -> launches: 32 members of 8 to 24 elements 3058 -> 2010 us, 8 members of 24 to
+            // 40 elements 1265 -> 850; 64 steps 6362 -> 6064, 3581 -> 3120.  The one launch per step: 1364 us
+            // from the graph, as many launched)
+            CUDA_TRY(enqueue(g, kGraphSteps, g->flip));
+            g->plain_runs++;
+            continue;
+        }
         if (!g->graph[g->flip]) {
             int rc = capture(g, kGraphSteps, g->flip, g->graph[g->flip]);
             if (rc) return rc;

@@ -17,6 +17,12 @@
 // of order 5 304.7 -> 291.9, 200^3 of order 4 1394.6 -> 1392.2, a group of 32 small boxes 36.7 -> 34.1.
 constexpr int kGraphSteps = 16;
 
+// Runs of kGraphSteps launched after a change (sources, receivers, model) before their graph is made: capturing
+// and instantiating one costs more than replaying saves over few steps.  The first 16 steps after a change,
+// graph -> launches: 12^3 elements of order 2 160 -> 103 us, 24^3 of order 4 231 -> 176, 40^3 400 -> 346; 128
+// steps 638 -> 597, 1200 -> 1173, 2550 -> 2514; beyond, the host's time counts.
+constexpr int kPlainRuns = 8;
+
 struct sem_solver {
     sem_mesh *mesh = nullptr;
     float dt = 0;

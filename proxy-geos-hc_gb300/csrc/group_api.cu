@@ -405,8 +405,8 @@ int sem_group_step(sem_group *g, int n_steps)
         if (form == SEM_GROUP_BRANCHES && !g->graph[g->flip] &&
             g->plain_runs + (n_steps - done) / kGraphSteps <= kPlainBranchRuns) {
             // (first 16 steps, graph -> launches: 32 members of 8 to 24 elements 3058 -> 2010 us, 8 members of 24 to
-            // 40 elements 1265 -> 850; 64 steps 6362 -> 6064, 3581 -> 3120.  The one launch per step: 1364 us
-            // from the graph, as many launched)
+            // 40 elements 1265 -> 850; 64 steps 6362 -> 6064, 3581 -> 3120.  The one launch per step is
+            // captured at once: 1364 us, 1382 with graphs of two steps)
             CUDA_TRY(enqueue(g, kGraphSteps, g->flip));
             g->plain_runs++;
             continue;

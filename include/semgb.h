@@ -385,8 +385,9 @@ int sem_adjoint_get_adjoint_traces(sem_adjoint *a, float *out);
  * caller owns, for callers that cannot allocate device memory while they step -- a host code
  * that gives all device memory to its own pool manager, or one whose time loop runs where
  * allocation is not allowed.  The call allocates nothing: the K.p accumulator lives in a fixed
- * array of 4,194,304 floats (16 MiB) in the library's device image, so the mesh may have at most 4,194,176 nodes; larger meshes are rejected with
- * SEM_ERR_ARG.  All buffers are device memory in the reference node numbering:
+ * array of 4,194,304 floats (16 MiB) in the library's device image, so the mesh may have at most
+ * 4,194,176 nodes; larger meshes are rejected with SEM_ERR_ARG.  All buffers are device memory in
+ * the reference node numbering:
  *   conn    int32 [n_elem][(order+1)^3] element-to-node map (as sem_mesh_get_connectivity gives);
  *           entries must lie in [0, n_nodes): one outside is skipped (read as 0, not scattered)
  *   p_cur   current level; sponge-damped in place when sponge factors are given

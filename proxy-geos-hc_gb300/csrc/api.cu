@@ -578,7 +578,8 @@ int sem_solver_create(sem_mesh *m, float dt, sem_solver **out)
     for (auto &p : s->d_p)
         if ((e = dalloc(&p, s->n_int)) != cudaSuccess || (e = cudaMemsetAsync(p, 0, s->n_int * 4, s->stream)) != cudaSuccess)
             return cleanup(SEM_ERR_OOM, std::string("pressure levels: ") + cudaGetErrorString(e));
-    if ((e = dalloc(&s->d_a, s->n_int)) != cudaSuccess || (e = cudaMemsetAsync(s->d_a, 0, s->n_int * 4, s->stream)) != cudaSuccess)
+    if ((e = dalloc(&s->d_a, s->n_int)) != cudaSuccess ||
+        (e = cudaMemsetAsync(s->d_a, 0, s->n_int * 4, s->stream)) != cudaSuccess)
         return cleanup(SEM_ERR_OOM, std::string("mass coefficient: ") + cudaGetErrorString(e));
     if ((e = dalloc(&s->d_ctr, 2)) != cudaSuccess || (e = cudaMemsetAsync(s->d_ctr, 0, 8, s->stream)) != cudaSuccess)
         return cleanup(SEM_ERR_CUDA, cudaGetErrorString(e));

@@ -208,7 +208,8 @@ int sem_batch_create(sem_mesh *m, float dt, int n_shots, sem_batch **out)
     for (auto &p : b->d_p)
         if ((e = dalloc(&p, n)) != cudaSuccess || (e = cudaMemsetAsync(p, 0, n * 4, b->stream)) != cudaSuccess)
             return cleanup(SEM_ERR_OOM, std::string("pressure levels: ") + cudaGetErrorString(e));
-    if ((e = dalloc(&b->d_a, b->n_int)) != cudaSuccess || (e = cudaMemsetAsync(b->d_a, 0, b->n_int * 4, b->stream)) != cudaSuccess)
+    if ((e = dalloc(&b->d_a, b->n_int)) != cudaSuccess ||
+        (e = cudaMemsetAsync(b->d_a, 0, b->n_int * 4, b->stream)) != cudaSuccess)
         return cleanup(SEM_ERR_OOM, cudaGetErrorString(e));
     if ((e = dalloc(&b->d_ctr, 2)) != cudaSuccess || (e = cudaMemsetAsync(b->d_ctr, 0, 8, b->stream)) != cudaSuccess)
         return cleanup(SEM_ERR_CUDA, cudaGetErrorString(e));

@@ -4,8 +4,8 @@
 // Two ways to advance them, both replayed from CUDA graphs of kGraphSteps steps (fewer: enqueued):
 //  - one launch (default where every member allows it: stencil pass, orders 1-4, direct form,
 //    default rounding): one pass launch per step over all members' CTAs (k_group.cu), sources
-//    launched once per run of steps and added by the passes between.  The members' tiles are cut along y into chunks of about the same number of
-//    planes, chosen for the whole group, and the longest CTAs come first in the launch;
+//    launched once per run of steps and added by the passes between.  The members' tiles are cut
+//    along y into chunks of about the same number of planes, chosen for the whole group, and the longest CTAs come first in the launch;
 //  - branches: the group stream forks into the members' streams, each branch holds that member's
 //    own steps (source, stencil pass), and the branches join back; largest member first.
 // Each member's results are bit for bit those of the member stepped alone, either way.  Members

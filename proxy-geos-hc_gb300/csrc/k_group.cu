@@ -4,8 +4,8 @@
 // Every member keeps its own levels, tensor maps and tiling; the launch's CTAs are the members'
 // tiles x y-chunks one after another (cta_member maps a CTA to its member), so the GPU's
 // scheduler fills SMs with whatever CTAs are left of any member, and a step of the whole group
-// is one launch (the pass, which also adds the next step's sources) instead of one per member.  A CTA runs the same code
-// as the single-box pass of its order (stencil_body.cuh), so each member's results are bit for
+// is one launch (the pass, which also adds the next step's sources) instead of one per member.  A CTA
+// runs the same code as the single-box pass of its order (stencil_body.cuh), so each member's results are bit for
 // bit those of the member stepped alone.  The CTA has kGroupThreads threads; at order 3 (three
 // warps) the fourth warp only takes part in the barriers.
 //
@@ -82,15 +82,25 @@ __global__ void __launch_bounds__(kGroupThreads, kGroupMinBlocks)
     }
     const NoClassTable none{};
     switch (order) {
-    case 1: stencil_cta<1, true, STENCIL_PLAIN, true, false, false, true>(rmap, wmap, pmap, amap, t, a, none, 0, bx, bz, chunk, step_off, inject != 0); break;
-    case 2: stencil_cta<2, true, STENCIL_PLAIN, true, false, false, true>(rmap, wmap, pmap, amap, t, a, none, 0, bx, bz, chunk, step_off, inject != 0); break;
-    case 3: stencil_cta<3, true, STENCIL_PLAIN, true, false, false, true>(rmap, wmap, pmap, amap, t, a, none, 0, bx, bz, chunk, step_off, inject != 0); break;
+    case 1:
+        stencil_cta<1, true, STENCIL_PLAIN, true, false, false, true>(rmap, wmap, pmap, amap, t, a, none, 0, bx, bz, chunk,
+                                                                      step_off, inject != 0);
+        break;
+    case 2:
+        stencil_cta<2, true, STENCIL_PLAIN, true, false, false, true>(rmap, wmap, pmap, amap, t, a, none, 0, bx, bz, chunk,
+                                                                      step_off, inject != 0);
+        break;
+    case 3:
+        stencil_cta<3, true, STENCIL_PLAIN, true, false, false, true>(rmap, wmap, pmap, amap, t, a, none, 0, bx, bz, chunk,
+                                                                      step_off, inject != 0);
+        break;
     default:
         if (shape == kTileSquare)
             stencil_cta<4, true, STENCIL_PLAIN, true, false, false, true, kSquareRW>(rmap, wmap, pmap, amap, t, a, none, 0,
                                                                                      bx, bz, chunk, step_off, inject != 0);
         else
-            stencil_cta<4, true, STENCIL_PLAIN, true, false, false, true>(rmap, wmap, pmap, amap, t, a, none, 0, bx, bz, chunk, step_off, inject != 0);
+            stencil_cta<4, true, STENCIL_PLAIN, true, false, false, true>(rmap, wmap, pmap, amap, t, a, none, 0, bx, bz,
+                                                                          chunk, step_off, inject != 0);
         break;
     }
 }

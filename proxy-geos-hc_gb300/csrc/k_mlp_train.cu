@@ -598,8 +598,9 @@ __device__ __forceinline__ void pack_param(const AdamArgs &o, int i, float p)
 }
 
 // sum over the slots b (in order) of part[b][i]: added to grad[i], or (kReduceAdam) the gradient of
-// one Adam step; kReduceGroups: so for each of ng consecutive groups of nb slots in turn.  The last block: the loss, lsum's 32 partial sums per slot as the quad leaders and
-// warps of a tile add them, slots in order, into *loss (added to it unless kReduceAdam).
+// one Adam step; kReduceGroups: so for each of ng consecutive groups of nb slots in turn.  The last
+// block: the loss, lsum's 32 partial sums per slot as the quad leaders and warps of a tile add them,
+// slots in order, into *loss (added to it unless kReduceAdam).
 enum ReduceMode { kReduceAdd, kReduceGroups, kReduceAdam };
 template <ReduceMode MODE>
 __global__ void __launch_bounds__(128) k_mlp_reduce(const float *part, const double *lsum, int nb, int ng, double n,

@@ -30,13 +30,6 @@ __device__ __forceinline__ uint16_t f2bf(float x)
     return *reinterpret_cast<const uint16_t *>(&b);
 }
 
-__device__ __forceinline__ float bf2f(uint16_t u)
-{
-    __nv_bfloat16 b;
-    *reinterpret_cast<uint16_t *>(&b) = u;
-    return __bfloat162float(b);
-}
-
 // two floats to BF16 (round to nearest even, as f2bf) in one conversion: lo in the low half
 __device__ __forceinline__ uint32_t pack_bf2(float lo, float hi)
 {

@@ -101,8 +101,9 @@ cudaError_t solver_enqueue_step(sem_solver *s, int c, cudaEvent_t *ev = nullptr,
 // n steps from level c with nothing between them.  side(k) (may be empty) gives step k's side buffers.
 cudaError_t solver_enqueue_run(sem_solver *s, int c, int n, const std::function<StepExtra(int)> &side = nullptr);
 void solver_invalidate_graphs(sem_solver *s);
-// Sources by device-layout node with explicit coefficients: p^n[node_k] += coef_k * wavelet_k[n].
+// The source table that the solver's launches read.
 semgb::SourceTable solver_sources(const sem_solver *s);
+// Sources by device-layout node with explicit coefficients: p^n[node_k] += coef_k * wavelet_k[n].
 int solver_set_raw_sources(sem_solver *s, int n_src, const int64_t *nodes, const float *coef, const float *wavelet,
                            int n_samples);
 // A field between the device layout (rows of nxp floats) and a host array in the reference

@@ -51,7 +51,10 @@ struct StencilBox {
     // 1: the last node along x (z) has no tile, the others fill whole tiles (see far_edges)
     int far_x = 0, far_z = 0;
     // Planes of a chunk divided among `parts` CTAs: first plane of part k, and the part of a plane.
-    __host__ __device__ static int part_begin(int planes, int parts, int k) { return (int)(((int64_t)planes * k + parts - 1) / parts); }
+    __host__ __device__ static int part_begin(int planes, int parts, int k)
+    {
+        return (int)(((int64_t)planes * k + parts - 1) / parts);
+    }
     __host__ __device__ static int part_of(int planes, int parts, int y) { return (int)((int64_t)y * parts / planes); }
 };
 

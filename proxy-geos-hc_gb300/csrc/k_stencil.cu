@@ -302,9 +302,10 @@ int stencil_tables_create(const Box &b, const Gll &g, const Geometry &geo, int n
     };
     // tile shape: the square order-4 tile for a single shot where it costs less, counting the
     // busiest slot's CTA-planes over the share of lanes on nodes (lanes past the box edge do the
-    // same work; measured on GB300, 64 x 16 against 32 x 32: 801^3 nodes 369.1 against 367.0
-    // Gnode-steps/s, 481^3 0.329 against 0.331 ms per step, 401^3 321.9 against 336.3, 345^3
-    // 0.145 against 0.130 ms, which this ranking orders the same way)
+    // same work).  It counts the tiles of the plain tiling, not of the far-edge form below, and a lead of 2o
+    // planes: right for most boxes, not for some of whole tiles plus one node.  us per step, 64 x 16
+    // against 32 x 32 (* chosen): 40^3 elements 18.8* / 20.0, 48^3 25.6 / 31.2*, 86^3 133.0 / 126.3*, 100^3
+    // 196.6 / 190.0*, 120^3 323.4* / 307.9, 200^3 1366* / 1375
     int sh = kTileDefault;
     if (b.order == 4 && nshot == 1) {
         if (shape == kTileSquare) {

@@ -148,6 +148,7 @@ inline int64_t stencil_tiles(int64_t n, int tile, bool far)
 // memory latencies before the march): small boxes, whose CTAs are all resident at once, keep the extra
 // tiles (40^3 elements of order 2: 4.7 us per step with them, 4.85 without; a group of 32 boxes of 8 to
 // 24 elements 34.1 against 42.7), larger ones drop them.
+// (Charged without a sponge too, where the edges need no work.)
 constexpr int kFarEdgeCost = 6;
 // Tables and tiling for a box (no device buffers yet).  Returns 0 or a cudaError_t.
 // nshot > 1: the many-shot form, levels holding nshot fields one after another (traces

@@ -58,4 +58,17 @@ struct sem_mesh {
     float *d_slow2 = nullptr;   // [n_int] when the node model is active (device layout)
     int32_t *d_conn = nullptr;  // [n_elem * npe], built on first use by the element kernel
     uint64_t model_version = 1;
+    // Writes of the model run here, behind the solvers' launches that read it (mesh_model_read).
+    cudaStream_t stream = nullptr;
 };
+
+// The work enqueued on s so far reads m's model: a model set later is written behind it.
+inline cudaError_t mesh_model_read(sem_mesh *m, cudaStream_t s)
+{
+    cudaEvent_t ev = nullptr;
+    cudaError_t e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventRecord(ev, s);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(m->stream, ev, 0);
+    if (ev) cudaEventDestroy(ev);
+    return e;
+}

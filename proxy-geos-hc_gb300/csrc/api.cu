@@ -420,13 +420,15 @@ int sem_mesh_create_box(int ex, int ey, int ez, float lx, float ly, float lz, in
     m->geo.g[1] = m->geo.detJ / (jz * jz);
     m->geo.g[2] = m->geo.detJ / (jy * jy);
     cudaGetDevice(&m->device);
-    cudaError_t e = dalloc(&m->d_vel, m->box.n_elem);
+    cudaError_t e = cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = dalloc(&m->d_vel, m->box.n_elem);
     if (e == cudaSuccess) {
         std::vector<float> v(m->box.n_elem, 1500.0f);  // SEMmesh::getModel
-        e = upload(m->d_vel, v.data(), v.size(), 0);
+        e = upload(m->d_vel, v.data(), v.size(), m->stream);
     }
     if (e != cudaSuccess) {
         dfree(m->d_vel);
+        if (m->stream) cudaStreamDestroy(m->stream);
         delete m;
         return fail(e == cudaErrorMemoryAllocation ? SEM_ERR_OOM : SEM_ERR_CUDA,
                     std::string("mesh allocation: ") + cudaGetErrorString(e));
@@ -442,6 +444,7 @@ int sem_mesh_destroy(sem_mesh *m)
     dfree(m->d_vel);
     dfree(m->d_slow2);
     dfree(m->d_conn);
+    if (m->stream) cudaStreamDestroy(m->stream);
     delete m;
     return SEM_OK;
 }
@@ -477,7 +480,7 @@ int sem_mesh_get_connectivity(sem_mesh *m, int32_t *conn)
 {
     GUARD_BEGIN
     if (!m || !conn) return fail(SEM_ERR_ARG, "NULL argument");
-    int rc = ensure_conn(m, 0);
+    int rc = ensure_conn(m, m->stream);
     if (rc) return rc;
     const size_t n = (size_t)m->box.n_elem * m->box.npe;
     CUDA_TRY(cudaMemcpy(conn, m->d_conn, n * sizeof(int32_t), cudaMemcpyDeviceToHost));
@@ -494,9 +497,7 @@ int sem_model_set_element_velocity(sem_mesh *m, const float *vel)
         if (!(vel[e] > 0) || !std::isfinite(vel[e]))
             return fail(SEM_ERR_ARG, "velocities must be positive and finite (element " +
                                          std::to_string(e) + ")");
-    // runs under way form their mass from the old model, on streams that the upload does not wait for
-    CUDA_TRY(cudaDeviceSynchronize());
-    CUDA_TRY(upload(m->d_vel, vel, m->box.n_elem, 0));
+    CUDA_TRY(upload(m->d_vel, vel, m->box.n_elem, m->stream));
     dfree(m->d_slow2);
     m->model_version++;
     return SEM_OK;
@@ -510,12 +511,11 @@ int sem_model_set_node_slowness2(sem_mesh *m, const float *s2)
     for (int64_t i = 0; i < m->box.n_nodes; i++)
         if (!(s2[i] > 0) || !std::isfinite(s2[i]))
             return fail(SEM_ERR_ARG, "squared slowness must be positive and finite");
-    CUDA_TRY(cudaDeviceSynchronize());  // as sem_model_set_element_velocity
     if (!m->d_slow2) {
         CUDA_TRY(dalloc(&m->d_slow2, m->box.n_int));
-        CUDA_TRY(cudaMemsetAsync(m->d_slow2, 0, m->box.n_int * 4, 0));
+        CUDA_TRY(cudaMemsetAsync(m->d_slow2, 0, m->box.n_int * 4, m->stream));
     }
-    CUDA_TRY(field_from_host(m->d_slow2, s2, m->box.nx, m->box.nxp, m->box.nz * m->box.ny, 0));
+    CUDA_TRY(field_from_host(m->d_slow2, s2, m->box.nx, m->box.nxp, m->box.nz * m->box.ny, m->stream));
     m->model_version++;
     return SEM_OK;
     GUARD_END
@@ -818,6 +818,7 @@ int solver_prepare(sem_solver *s, int64_t n_new)
         CUDA_TRY(launch_mass(s->d_a, m->d_slow2 ? nullptr : m->d_vel, m->d_slow2, m->box.ex, m->box.ey,
                              m->box.ez, m->box.order, m->box.nxp, s->d_w, m->geo.detJ,
                              (double)s->dt * s->dt, s->stream));
+        CUDA_TRY(mesh_model_read(m, s->stream));
         s->a_version = m->model_version;
     }
     if (kern == SEM_KERNEL_ELEMENT) {
@@ -844,6 +845,7 @@ int solver_prepare(sem_solver *s, int64_t n_new)
             // detJ grouped as computeB forms it (SEMQkGLIntegrals.hpp:316-318)
             const double detJ = std::fabs((0.5 * b.lx / b.ex) * ((0.5 * b.lz / b.ez) * (0.5 * b.ly / b.ey)));
             CUDA_TRY(launch_mass_ref(s->d_mref, m->d_vel, b.ex, b.ey, b.ez, b.order, b.nxp, s->d_w, detJ, s->stream));
+            CUDA_TRY(mesh_model_read(m, s->stream));
             s->mref_version = m->model_version;
         }
         if (s->upd_rec_version != s->rec_version) {

@@ -118,6 +118,7 @@ int prepare(sem_batch *b, int64_t n_new)
     if (b->a_version != m->model_version) {
         CUDA_TRY(launch_mass(b->d_a, m->d_slow2 ? nullptr : m->d_vel, m->d_slow2, m->box.ex, m->box.ey, m->box.ez,
                              m->box.order, m->box.nxp, b->d_w, m->geo.detJ, (double)b->dt * b->dt, b->stream));
+        CUDA_TRY(mesh_model_read(m, b->stream));
         b->a_version = m->model_version;
     }
     if (stencil_bind(*b->st, b->d_p[0], b->d_p[1], b->d_a) != 0)
